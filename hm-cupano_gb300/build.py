@@ -44,7 +44,7 @@ UNITS = {
 }
 RDC_UNITS = [u for u, extra in UNITS.items() if "-rdc=true" in extra]
 HEADERS = ["hmp_plan.h", "hmp_copyplan.h", "hmp_device.cuh", "hmp_kernels.h", "hmp_blend.cuh", "hmp_admission.h",
-           "hmp_pyramid_kernels.cuh"]
+           "hmp_pyramid_kernels.cuh", "hmp_ordered_sum.h"]
 
 
 def nvcc() -> str:
