@@ -36,6 +36,7 @@ UNITS = {
     "hmp_server.cpp": [],
     "hmp_control_dir.cpp": [],
     "hmp_generic.cu": ["-fmad=false"],
+    "hmp_rgb.cu": ["-fmad=false"],
     "hmp_batch.cpp": [],
     "hmp_stabilize.cu": ["-fmad=false"],
     # Device-side (tail) launches need relocatable device code; only this unit has it, since it

@@ -8,11 +8,12 @@ namespace hmp {
 void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
   cp = CopyPlan{};
   const int L = p.levels, n = p.n;
-  if (L < 2 || p.filter != HMP_FILTER_REFBOX || p.generic() || !p.canvas_plane_used) return;
+  const bool rgb = p.rgb8();
+  if (L < 2 || p.filter != HMP_FILTER_REFBOX || p.generic() || (!rgb && !p.canvas_plane_used)) return;
   const bool two = p.rule == kRuleTwo;
   // Two images: the minimised strip only, whose content lines up with the canvas (image 1's table
   // at column 0); three or more: any blend region.
-  if (two ? (!p.minimized || p.strip_shift != 0) : n < 3) return;
+  if (!rgb && (two ? (!p.minimized || p.strip_shift != 0) : n < 3)) return;
   const int bw = p.lw[0], bh = p.lh[0];
   if (bw <= 0 || bh <= 0 || int(p.mask0.size()) != bw * bh || int(p.slots.size()) != n) return;
   // Level-(L-1) pixel q covers level-0 block q of edge G; per block: the label if uniform, and per
@@ -38,7 +39,7 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
   std::vector<uint8_t> all_valid(size_t(n) * nb, 1), any_valid(size_t(n) * nb, 0);
   std::vector<uint16_t> max_sx(size_t(n) * nb, 0), max_sy(size_t(n) * nb, 0);
   std::vector<uint8_t> img2_any(two ? nb : 0, 0);  // two images: any entry of image 2 in the block
-  for (int k = 0; k < n; ++k) {
+  for (int k = 0; !rgb && k < n; ++k) {
     const GatherPlane& s = p.slots[k];
     uint8_t* av = &all_valid[size_t(k) * nb];
     uint8_t* an = &any_valid[size_t(k) * nb];
@@ -73,6 +74,7 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
     }
   }
 
+  // RGB8: all_valid stays set (every pixel counts) and no block is classed empty.
   // pyr_fine's blocks over the write rect (blend coordinates), and each block's support.
   const int wx0 = p.write.x - p.blend.x, wy0 = p.write.y - p.blend.y;
   const int wx1 = wx0 + p.write.w, wy1 = wy0 + p.write.h;
@@ -97,7 +99,7 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
       // 1 selects slot 0 (image 1) and 0 slot 1 (image 2, or image 1 where image 2 has no table).
       const int label = lab[size_t(sy0) * gx + sx0];
       const int k = two ? (label == 1 ? 0 : (label == 0 ? 1 : n)) : label;
-      bool copy = k < n, empty = true;
+      bool copy = k < n, empty = !rgb;
       for (int by = sy0; by <= sy1; ++by)
         for (int bx = sx0; bx <= sx1; ++bx) {
           const size_t b = size_t(by) * gx + bx;
@@ -197,6 +199,41 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
   cp.support_shift = L - 1;
   cp.usable = cp.copy_blocks + cp.empty_blocks > 0 && ndx < 0x8000 && ndy < 0x8000 && ncx < 0x8000 &&
               ncy < 0x8000 && cp.nfx < 0x8000 && cp.nfy < 0x8000;
+}
+
+void rgb_canvas_plane(Plan& p, const CopyPlan& c) {
+  if (!c.usable) return;
+  GatherPlane& g = p.canvas;
+  const size_t px = size_t(p.canvas_w) * p.canvas_h;
+  if (!p.canvas_plane_used) {
+    g.rect = Rect{0, 0, p.canvas_w, p.canvas_h};
+    g.owner.assign(px, kNoOwner);
+    g.map.assign(px, kNoEntry);
+    p.canvas_plane_used = true;
+    p.canvas_opaque = false;
+  }
+  const int wx0 = p.write.x - p.blend.x, wy0 = p.write.y - p.blend.y;
+  const int wx1 = wx0 + p.write.w, wy1 = wy0 + p.write.h;
+  for (int j = 0; j < c.nfy; ++j)
+    for (int i = 0; i < c.nfx; ++i) {
+      if (c.block_class[size_t(j) * c.nfx + i] != kBlockCopy) continue;
+      const int x0 = std::max(c.fx0 + 64 * i, wx0), x1 = std::min(c.fx0 + 64 * i + 64, wx1);
+      const int y0 = std::max(c.fy0 + 16 * j, wy0), y1 = std::min(c.fy0 + 16 * j + 16, wy1);
+      const int label = p.mask0[size_t(y0) * p.lw[0] + x0];
+      const GatherPlane& s = p.slots[p.rule == kRuleTwo ? (label == 1 ? 0 : 1) : label];
+      for (int y = y0; y < y1; ++y)
+        for (int x = x0; x < x1; ++x) {
+          const size_t d = size_t(y + p.blend.y) * p.canvas_w + (x + p.blend.x);
+          if (!s.rect.contains(x, y)) {
+            g.owner[d] = kNoOwner;
+            g.map[d] = kNoEntry;
+            continue;
+          }
+          const size_t q = size_t(y - s.rect.y) * s.rect.w + (x - s.rect.x);
+          g.owner[d] = s.map[q] == kNoEntry ? kNoOwner : (s.owner.empty() ? uint8_t(s.default_owner) : s.owner[q]);
+          g.map[d] = s.map[q];
+        }
+    }
 }
 
 }  // namespace hmp

@@ -30,6 +30,11 @@
 //     by the gather over the blend region, for the pixels it copies and those outside the write
 //     rect, and by pyr_fine for the pyramid-block pixels inside a support, the only others a
 //     support holds; any alpha 0 gates on the fallback launches, which recompute the write rect).
+// RGB8 frames have no alpha and no validity: an unmapped pixel is 0 and counts like any other, so a
+// block is a copy wherever the labels of its supports are one image's, the copied pixel is that
+// slot's level-0 pixel (0 where it has none), and nothing is checked per frame. The canvas plane
+// takes those entries from the slots (rgb_canvas_plane), for any blend region.
+//
 // The pyramid then runs only where it is needed: pyr_fine over the pyramid blocks, pyr_coarse over
 // the level-1 tiles those read (R^1), pyr_down over the level-0 tiles whose levels either reads.
 #pragma once
@@ -66,7 +71,11 @@ struct CopyPlan {
 // Leaves out.usable false where they do not apply: two images without the minimised strip (or with
 // image 1's table off column 0, which shifts the strip's content against the canvas), N-image
 // stitchers of two images, fewer than two levels, the Binomial5 filter (its 5-tap sums are not
-// short dyadic fractions), and non-RGBA8 pixels.
+// short dyadic fractions), and float pixels. RGB8: any blend region of two or more levels.
 void plan_copy_blocks(const Plan& p, int tile_down, int tile_coarse, CopyPlan& out);
+
+// RGB8: writes the copy blocks' slot entries into the canvas plane (made here where the
+// configuration has none).
+void rgb_canvas_plane(Plan& p, const CopyPlan& c);
 
 }  // namespace hmp

@@ -197,11 +197,11 @@ __global__ void __launch_bounds__(256, 6) canvas_gather_kernel(const __grid_cons
 // Resolves one plane's packed entries (raw.map) for the frames' geometry (res, same layout):
 // owner o < n and (sx, sy) inside image o give o << 29 | (sy * pitch / 4 + sx); anything else
 // kOffZero, or kOffOpaque under the soft-seam rule when the owner is valid and sx is not the
-// 65535 sentinel. (Frames hold fewer than kOffMask - 1 pixels, so no offset meets a fill code.)
+// 65535 sentinel. rgb: byte offsets of three-byte pixels. (Frames hold fewer than kOffMask - 1 pixels, so no offset meets a fill code.)
 __global__ void __launch_bounds__(kSegPixels) resolve_plane_kernel(const __grid_constant__ PlaneDev raw, uint32_t* res,
                                                                    uint8_t* seg_owner, int seg_pitch,
                                                                    const __grid_constant__ SrcSet S, int n, int opaque,
-                                                                   const __grid_constant__ SkipMap skip) {
+                                                                   int rgb, const __grid_constant__ SkipMap skip) {
   // One CTA per 256-pixel row segment, the gather's unit.
   const int x = blockIdx.x * kSegPixels + threadIdx.x, y = blockIdx.y;
   uint32_t r = kOffZero;  // pixels past the plane's width read as fills
@@ -212,7 +212,8 @@ __global__ void __launch_bounds__(kSegPixels) resolve_plane_kernel(const __grid_
     const int sx = int(e & 0xFFFFu), sy = int(e >> 16);
     if (o < n) {
       if (sx < S.w[o] && sy < S.h[o])
-        r = (uint32_t(o) << kOwnerShift) | (uint32_t(sy) * uint32_t(S.pitch[o] / 4) + uint32_t(sx));
+        r = (uint32_t(o) << kOwnerShift) | (rgb ? uint32_t(sy) * uint32_t(S.pitch[o]) + 3u * uint32_t(sx)
+                                                : uint32_t(sy) * uint32_t(S.pitch[o] / 4) + uint32_t(sx));
       else if (opaque && sx != 0xFFFF)
         r = kOffOpaque;
     }
@@ -256,10 +257,10 @@ __global__ void __launch_bounds__(kSegPixels) resolve_plane_kernel(const __grid_
 }  // namespace
 
 cudaError_t launch_resolve_plane(const PlaneDev& raw, uint32_t* res, uint8_t* seg_owner, int seg_pitch, const SrcSet& S,
-                                 int n, bool opaque, const SkipMap& skip, cudaStream_t stream) {
+                                 int n, bool opaque, bool rgb, const SkipMap& skip, cudaStream_t stream) {
   if (raw.w <= 0 || raw.h <= 0) return cudaSuccess;
   resolve_plane_kernel<<<dim3((raw.w + kSegPixels - 1) / kSegPixels, raw.h), kSegPixels, 0, stream>>>(
-      raw, res, seg_owner, seg_pitch, S, n, opaque ? 1 : 0, skip);
+      raw, res, seg_owner, seg_pitch, S, n, opaque ? 1 : 0, rgb ? 1 : 0, skip);
   return cudaGetLastError();
 }
 

@@ -1,8 +1,9 @@
-// hmp_generic.cu -- the stitch for the reference's other pixel pipelines: uchar3, float4 and float3
-// (CudaStitchPano*<uchar3, float3>, <float4, float4>, <float3, float3>; src/pano/cudaPano3_test.cpp,
-// tests/testCudaBlend.cpp). RGBA8 runs the fused kernels of hmp_gather.cu / hmp_pyramid.cu; these
-// pipelines are used by the reference's tests and tools rather than its video path, so they run
-// plain level-by-level kernels over float4 level buffers in HBM, with the reference's arithmetic:
+// hmp_generic.cu -- the stitch for the reference's float pixel pipelines: float4 and float3
+// (CudaStitchPano*<float4, float4>, <float3, float3>; src/pano/cudaPano3_test.cpp,
+// tests/testCudaBlend.cpp). RGBA8 runs the fused kernels of hmp_gather.cu / hmp_pyramid.cu and RGB8
+// those of hmp_rgb.cu; the float pipelines are used by the reference's tests and tools rather than
+// its video path, so they run plain level-by-level kernels over float4 level buffers in HBM, with the
+// reference's arithmetic:
 //   level 0   per image, the remap over the blend region (cudaRemap.cu:60-123): the source pixel if
 //             the table entry is inside the frame, else 0 (4 channels: alpha 255 under the soft-seam
 //             rule for an entry that is not the 65535 sentinel)
@@ -14,8 +15,8 @@
 //   blend     4 channels: blend_level / blend_level0 (the reference rules, alpha tests included);
 //             3 channels: two images m*a + (1-m)*b (cudaBlend.cu:520-576), three m1*v1 + m2*v2 +
 //             m3*v3 (cudaBlend3.cu:376-531), N the mask normalised by its sum (cudaBlendN.cu:199-288)
-//   reconstruct  up(R^(l+1)) + blend^l; level 0 written into the canvas's write rect, packed by
-//             truncation for uint8 pipelines, as is for float ones (cudaMakeFull.cu:241-258)
+//   reconstruct  up(R^(l+1)) + blend^l; level 0 written into the canvas's write rect, as is
+//             (cudaMakeFull.cu:241-258)
 // and the canvas outside the write rect (or all of it for the hard seam) copied from the canvas
 // plane's entries. Compiled with -fmad=false, like the fused kernels.
 #include <cuda_runtime.h>
@@ -26,45 +27,32 @@
 namespace hmp {
 namespace {
 
-// Pixel of C channels, uint8 or float samples (F), at byte address p.
-template <int C, bool F>
+// Pixel of C float channels at byte address p.
+template <int C>
 struct Px {
-  static constexpr int kBytes = C * (F ? 4 : 1);
+  static constexpr int kBytes = C * 4;
   __device__ __forceinline__ static float4 load(const char* p) {
-    if constexpr (F) {
-      const float* f = reinterpret_cast<const float*>(p);
-      return make_float4(f[0], f[1], f[2], C == 4 ? f[3] : 0.f);
-    } else {
-      const unsigned char* u = reinterpret_cast<const unsigned char*>(p);
-      return make_float4(float(u[0]), float(u[1]), float(u[2]), C == 4 ? float(u[3]) : 0.f);
-    }
+    const float* f = reinterpret_cast<const float*>(p);
+    return make_float4(f[0], f[1], f[2], C == 4 ? f[3] : 0.f);
   }
   __device__ __forceinline__ static void store(char* p, const float4 v) {
-    if constexpr (F) {
-      float* f = reinterpret_cast<float*>(p);
-      f[0] = v.x;
-      f[1] = v.y;
-      f[2] = v.z;
-      if (C == 4) f[3] = v.w;
-    } else {
-      unsigned char* u = reinterpret_cast<unsigned char*>(p);
-      u[0] = pack_u8(v.x);
-      u[1] = pack_u8(v.y);
-      u[2] = pack_u8(v.z);
-      if (C == 4) u[3] = pack_u8(v.w);
-    }
+    float* f = reinterpret_cast<float*>(p);
+    f[0] = v.x;
+    f[1] = v.y;
+    f[2] = v.z;
+    if (C == 4) f[3] = v.w;
   }
 };
 
 // Source pixel for (owner o, packed entry e) in frame b, or the remap's fill.
-template <int C, bool F>
+template <int C>
 __device__ __forceinline__ float4 fetch(const SrcSet& S, int n, int o, uint32_t e, int b, bool opaque) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   if (o >= n) return v;
   const int sx = int(e & 0xFFFFu), sy = int(e >> 16);
   if (sx < S.w[o] && sy < S.h[o]) {
     const char* base = reinterpret_cast<const char*>(S.ptr[o]) + b * S.bstride[o] + (long long)sy * S.pitch[o];
-    return Px<C, F>::load(base + (long long)sx * Px<C, F>::kBytes);
+    return Px<C>::load(base + (long long)sx * Px<C>::kBytes);
   }
   if (C == 4 && opaque && sx != 0xFFFF) v.w = 255.f;
   return v;
@@ -153,7 +141,7 @@ __device__ __forceinline__ float4 blend_rgb(int n, const float4* L, const float*
   return r;
 }
 
-template <int C, bool F>
+template <int C>
 __global__ void gen_level0_kernel(const __grid_constant__ GenArgs a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   const int k = int(blockIdx.z) % a.n, b = int(blockIdx.z) / a.n;
@@ -167,7 +155,7 @@ __global__ void gen_level0_kernel(const __grid_constant__ GenArgs a) {
     e = P.map[(long long)ry * P.map_pitch + rx];
     if (P.owner != nullptr) o = int(P.owner[(long long)ry * P.owner_pitch + rx]);
   }
-  a.G[k][0][((long long)b * lh0 + y) * lw0 + x] = fetch<C, F>(a.S, a.n, o, e, b, a.opaque != 0);
+  a.G[k][0][((long long)b * lh0 + y) * lw0 + x] = fetch<C>(a.S, a.n, o, e, b, a.opaque != 0);
 }
 
 template <int C>
@@ -208,7 +196,7 @@ __global__ void gen_down_kernel(const __grid_constant__ GenArgs a, int l) {
 
 // Level l: the Laplacians of every image, their blend and the reconstruction (into `rout`, or into
 // the canvas's write rect at level 0).
-template <int C, bool F, int RULE, int NMAX>
+template <int C, int RULE, int NMAX>
 __global__ void gen_up_kernel(const __grid_constant__ GenArgs a, int l, const float4* rnext, float4* rout) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, b = blockIdx.z;
   const int w = a.lw[l], h = a.lh[l];
@@ -260,11 +248,11 @@ __global__ void gen_up_kernel(const __grid_constant__ GenArgs a, int l, const fl
   }
   if (x < a.wx0 || x >= a.wx1 || y < a.wy0 || y >= a.wy1) return;
   char* row = reinterpret_cast<char*>(a.C.ptr) + b * a.C.bstride + (long long)(y + a.cy_off) * a.C.pitch;
-  Px<C, F>::store(row + (long long)(x + a.cx_off) * Px<C, F>::kBytes, r);
+  Px<C>::store(row + (long long)(x + a.cx_off) * Px<C>::kBytes, r);
 }
 
 // Canvas pixels outside the skipped rect from the canvas plane's packed entries.
-template <int C, bool F>
+template <int C>
 __global__ void gen_canvas_kernel(const __grid_constant__ GatherArgs g, int opaque) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, b = blockIdx.z;
   if (x >= g.C.w) return;
@@ -272,51 +260,45 @@ __global__ void gen_canvas_kernel(const __grid_constant__ GatherArgs g, int opaq
   const PlaneDev& P = g.P;
   const int o = P.owner ? int(P.owner[(long long)y * P.owner_pitch + x]) : P.default_owner;
   const uint32_t e = P.map[(long long)y * P.map_pitch + x];
-  const float4 v = fetch<C, F>(g.S, g.n_owners, o, e, b, opaque != 0);
+  const float4 v = fetch<C>(g.S, g.n_owners, o, e, b, opaque != 0);
   char* row = reinterpret_cast<char*>(g.C.ptr) + b * g.C.bstride + (long long)y * g.C.pitch;
-  Px<C, F>::store(row + (long long)x * Px<C, F>::kBytes, v);
+  Px<C>::store(row + (long long)x * Px<C>::kBytes, v);
 }
 
 dim3 grid_of(int w, int h, int z) { return dim3((w + 255) / 256, h, z); }
 
-template <int C, bool F>
+template <int C>
 cudaError_t run_pyramid(const GenArgs& a, int rule, int batch, float4* const* r, cudaStream_t s) {
   const int L = a.levels;
-  gen_level0_kernel<C, F><<<grid_of(a.lw[0], a.lh[0], batch * a.n), 256, 0, s>>>(a);
+  gen_level0_kernel<C><<<grid_of(a.lw[0], a.lh[0], batch * a.n), 256, 0, s>>>(a);
   for (int l = 1; l < L; ++l) gen_down_kernel<C><<<grid_of(a.lw[l], a.lh[l], batch * a.n), 256, 0, s>>>(a, l);
   for (int l = L - 1; l >= 0; --l) {
     const float4* rnext = l + 1 < L ? r[(l + 1) & 1] : nullptr;
     float4* rout = l > 0 ? r[l & 1] : nullptr;
     const dim3 grid = grid_of(a.lw[l], a.lh[l], batch);
     if (rule == kRuleTwo)
-      gen_up_kernel<C, F, kRuleTwo, 2><<<grid, 256, 0, s>>>(a, l, rnext, rout);
+      gen_up_kernel<C, kRuleTwo, 2><<<grid, 256, 0, s>>>(a, l, rnext, rout);
     else if (rule == kRuleThree)
-      gen_up_kernel<C, F, kRuleThree, 3><<<grid, 256, 0, s>>>(a, l, rnext, rout);
+      gen_up_kernel<C, kRuleThree, 3><<<grid, 256, 0, s>>>(a, l, rnext, rout);
     else
-      gen_up_kernel<C, F, kRuleNway, kDevMaxImages><<<grid, 256, 0, s>>>(a, l, rnext, rout);
+      gen_up_kernel<C, kRuleNway, kDevMaxImages><<<grid, 256, 0, s>>>(a, l, rnext, rout);
   }
   return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_generic_pyramid(const GenArgs& a, int channels, bool is_float, int rule, int batch,
-                                   float4* const* r, cudaStream_t stream) {
-  if (channels == 4) return is_float ? run_pyramid<4, true>(a, rule, batch, r, stream)
-                                     : run_pyramid<4, false>(a, rule, batch, r, stream);
-  return is_float ? run_pyramid<3, true>(a, rule, batch, r, stream) : run_pyramid<3, false>(a, rule, batch, r, stream);
+cudaError_t launch_generic_pyramid(const GenArgs& a, int channels, int rule, int batch, float4* const* r,
+                                   cudaStream_t stream) {
+  return channels == 4 ? run_pyramid<4>(a, rule, batch, r, stream) : run_pyramid<3>(a, rule, batch, r, stream);
 }
 
-cudaError_t launch_generic_canvas(const GatherArgs& g, int channels, bool is_float, bool opaque, cudaStream_t stream) {
+cudaError_t launch_generic_canvas(const GatherArgs& g, int channels, bool opaque, cudaStream_t stream) {
   const dim3 grid = grid_of(g.C.w, g.C.h, g.batch);
-  if (channels == 4 && is_float)
-    gen_canvas_kernel<4, true><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
-  else if (channels == 4)
-    gen_canvas_kernel<4, false><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
-  else if (is_float)
-    gen_canvas_kernel<3, true><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
+  if (channels == 4)
+    gen_canvas_kernel<4><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
   else
-    gen_canvas_kernel<3, false><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
+    gen_canvas_kernel<3><<<grid, 256, 0, stream>>>(g, opaque ? 1 : 0);
   return cudaGetLastError();
 }
 

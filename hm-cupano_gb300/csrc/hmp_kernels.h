@@ -41,7 +41,7 @@ struct PyrArgs {
   const uint8_t* mask0;                   // level-0 weight value (two-image) or label, blend coords
   int mask0_pitch;
   const float* maskL[kDevMaxLevels];      // level l >= 1: [lh][lw][K]
-  const uint8_t* hotL[kDevMaxLevels];     // N-way rule, level l >= 1: [lh][lw] mask class
+  const uint8_t* hotL[kDevMaxLevels];     // N-way rule and RGB8, level l >= 1: [lh][lw] mask class
   int K;
   int opaque;
   int tile;  // tile edge (level 0 for pyr_down, level 1 for pyr_coarse)
@@ -93,7 +93,17 @@ cudaError_t launch_dump_blend2(const float4* l0, const float4* l1, const float* 
 cudaError_t launch_dump_recon(const float4* lo, int lw, int lh, const float4* bl, int w, int h, float4* out, int batch,
                               cudaStream_t stream);
 
-// Level-by-level stitch of the uchar3 / float4 / float3 pipelines (hmp_generic.cu).
+// The stitch of RGB8 frames (hmp_rgb.cu): PyrArgs with float4 levels (w unused), mask classes for every
+// rule, and slots_cap / coarse_cap / fine_cap for any number of images. packed: the canvas plane's
+// packed entries (frames past the resolved offsets' range), skip blocks from `skip`.
+struct SkipMap;
+cudaError_t rgb_init();
+cudaError_t launch_rgb_gather(const GatherArgs& a, bool packed, const SkipMap& skip, cudaStream_t stream);
+cudaError_t launch_rgb_down(const PyrArgs& a, dim3 grid, cudaStream_t stream);
+cudaError_t launch_rgb_coarse(const PyrArgs& a, int rule, dim3 grid, size_t smem, cudaStream_t stream);
+cudaError_t launch_rgb_fine(const PyrArgs& a, int rule, dim3 grid, cudaStream_t stream);
+
+// Level-by-level stitch of the float4 / float3 pipelines (hmp_generic.cu).
 struct GenArgs {
   SrcSet S;  // frames; ptr is the first pixel of any sample type
   PlaneDev slot[kDevMaxImages];
@@ -112,10 +122,10 @@ struct GenArgs {
   int cx_off, cy_off;      // canvas = blend + offset
 };
 // r[0], r[1]: reconstruction buffers of level-1 size (levels alternate between them).
-cudaError_t launch_generic_pyramid(const GenArgs& a, int channels, bool is_float, int rule, int batch,
-                                   float4* const* r, cudaStream_t stream);
+cudaError_t launch_generic_pyramid(const GenArgs& a, int channels, int rule, int batch, float4* const* r,
+                                   cudaStream_t stream);
 // The canvas outside g's skip rect from the raw (packed) canvas plane g.P.
-cudaError_t launch_generic_canvas(const GatherArgs& g, int channels, bool is_float, bool opaque, cudaStream_t stream);
+cudaError_t launch_generic_canvas(const GatherArgs& g, int channels, bool opaque, cudaStream_t stream);
 int generic_launches(int levels, bool canvas);
 
 // One-time attribute setup (dynamic shared memory limits). Call before capture.
@@ -137,8 +147,9 @@ struct SkipMap {
   int pitch, x0, y0, nx, ny;
   int wr_x0, wr_y0, wr_x1, wr_y1;  // canvas coordinates, end exclusive
 };
+// rgb: offsets are bytes of three-byte pixels (else whole 4-byte pixels).
 cudaError_t launch_resolve_plane(const PlaneDev& raw, uint32_t* res, uint8_t* seg_owner, int seg_pitch, const SrcSet& S,
-                                 int n, bool opaque, const SkipMap& skip, cudaStream_t stream);
+                                 int n, bool opaque, bool rgb, const SkipMap& skip, cudaStream_t stream);
 
 // copy_blocks: the plane holds copy-block skips (kOffSkip) or the call checks source alpha.
 cudaError_t launch_canvas_gather(const GatherArgs& a, bool copy_blocks, cudaStream_t stream);

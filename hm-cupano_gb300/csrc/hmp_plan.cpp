@@ -317,7 +317,7 @@ int build_plan(const hmp_config& c, Plan& p, std::string& m) {
     seam_owner_plane(c, p);
     p.canvas_plane_used = true;
     p.canvas_opaque = false;
-  } else if (p.rule != kRuleTwo && p.n >= 3 && p.levels >= 2 && p.filter == HMP_FILTER_REFBOX && !p.generic()) {
+  } else if (p.rule != kRuleTwo && p.n >= 3 && p.levels >= 2 && p.filter == HMP_FILTER_REFBOX && !p.generic() && !p.rgb8()) {
     // Three images, or N without a minimised blend region: the pyramid covers the whole canvas,
     // and the seam-selected plane serves the copy blocks, where the pyramid's result is the
     // label's pixel (hmp_copyplan.h).
@@ -409,13 +409,17 @@ int build_plan(const hmp_config& c, Plan& p, std::string& m) {
     p.mask_levels[l] = nxt;
     cur.swap(nxt);
   }
-  // The N-way kernels pick from the class alone unless the weights are fractional.
+  // The N-way and RGB8 kernels pick from the class alone unless the weights are fractional.
   p.mask_hot.assign(p.levels, {});
-  for (int l = 1; p.rule == kRuleNway && l < p.levels; ++l) {
+  for (int l = 1; (p.rule == kRuleNway || p.rgb8()) && l < p.levels; ++l) {
     const std::vector<float>& wts = p.mask_levels[l];
     std::vector<uint8_t>& h = p.mask_hot[l];
     h.resize(size_t(p.lw[l]) * p.lh[l]);
     for (size_t i = 0; i < h.size(); ++i) {
+      if (p.rule == kRuleTwo) {  // one value, the weight of image 1
+        h[i] = wts[i] == 1.0f ? 0 : (wts[i] == 0.0f ? 1 : uint8_t(kHotFrac));
+        continue;
+      }
       int hot = kHotNone;
       for (int k = 0; k < K && hot != kHotFrac; ++k) {
         const float w = wts[i * K + k];

@@ -24,9 +24,9 @@ constexpr int kMaxLevels = 7;          // levels one fused pyramid pass supports
 
 enum BlendRule : int { kRuleNway = 1, kRuleTwo = 2, kRuleThree = 3 };
 
-// Mask class of an N-way pixel at level l >= 1 (values shared with the kernels): 0..n-1 = the
-// image whose weight is 1 while the others are 0; kHotNone = every weight 0; kHotFrac = any other
-// weights (the blend then reads the K mask values).
+// Mask class of a pixel at level l >= 1 (values shared with the kernels): 0..n-1 = the image whose
+// weight is 1 while the others are 0; kHotNone = every weight 0; kHotFrac = any other weights (the
+// blend then reads the K mask values).
 enum MaskHot : uint8_t { kHotNone = 0xFE, kHotFrac = 0xFF };
 
 struct Rect {
@@ -56,8 +56,10 @@ struct Plan {
   int mask_k = 1;        // mask channels of the pyramid blend
   int channels = 4;      // 4 (RGBA) or 3 (RGB)
   bool pixel_float = false;  // float samples (HMP_PIXEL_F32) instead of uint8
-  // Everything but RGBA8 runs the level-by-level kernels (hmp_generic.cu).
-  bool generic() const { return channels != 4 || pixel_float; }
+  // Float samples run the level-by-level kernels (hmp_generic.cu), RGB8 its own fused ones
+  // (hmp_rgb.cu).
+  bool generic() const { return pixel_float; }
+  bool rgb8() const { return channels == 3 && !pixel_float; }
   int pixel_bytes() const { return channels * (pixel_float ? 4 : 1); }
   bool minimized = false;
   bool slot_opaque = true;    // soft-seam rule: out-of-range, non-sentinel entries give alpha 255
@@ -70,7 +72,7 @@ struct Plan {
   std::vector<GatherPlane> slots;   // n, blend coordinates
   std::vector<uint8_t> mask0;       // blend.w * blend.h: two-image weight value or label
   std::vector<std::vector<float>> mask_levels;  // levels >= 1: lw*lh*mask_k floats
-  std::vector<std::vector<uint8_t>> mask_hot;   // N-way rule, levels >= 1: lw*lh MaskHot classes
+  std::vector<std::vector<uint8_t>> mask_hot;   // N-way rule and RGB8, levels >= 1: lw*lh MaskHot classes
   std::vector<int> lw, lh;          // level dims
   // Two images, minimised: the blend strip's content is the canvas shifted by image 1's table
   // column (the reference copies full1 / full2 out of the canvas at that offset).

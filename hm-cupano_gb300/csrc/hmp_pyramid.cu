@@ -229,6 +229,7 @@ cudaError_t kernels_init() {
   set_coarse_attrs<float4, 32>();
   set_coarse_attrs<half4, 32>();
   fallback_init();
+  rgb_init();
   return cudaGetLastError();
 }
 

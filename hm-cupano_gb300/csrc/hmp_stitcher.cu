@@ -166,7 +166,8 @@ struct hmp_stitcher {
   int launches = 0;
   hmp::SrcSet last_src{};  // frames of the last process(), for the pyramid dump
   bool have_last = false;
-  bool generic = false;    // uchar3 / float4 / float3 pixels: the level-by-level kernels
+  bool generic = false;    // float4 / float3 pixels: the level-by-level kernels
+  bool rgb = false;        // uchar3 pixels: the kernels of hmp_rgb.cu
   float4* G0[hmp::kDevMaxImages]{};  // generic: level 0 per slot
   float4* Rg[2]{};                   // generic: reconstruction buffers (level-1 size)
   // Optional per-kernel event timing (hmp_stitcher_set_timing).
@@ -321,8 +322,14 @@ struct hmp_stitcher {
   hmp_status setup() {
     hmp::Plan& p = plan;
     generic = p.generic();
+    rgb = p.rgb8();
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return cuda_status(e, "cudaGetDevice");
+    hmp::CopyPlan cps[2];  // down tiles of 32 and 64 pixels
+    if (rgb) {  // the copy blocks' entries go into the canvas plane before it is uploaded
+      plan_copies(cps);
+      hmp::rgb_canvas_plane(p, cps[1].usable ? cps[1] : cps[0]);
+    }
     e = hmp::kernels_init();
     if (e != cudaSuccess) return cuda_status(e, "kernel setup");
     if (p.canvas_plane_used) {
@@ -432,7 +439,8 @@ struct hmp_stitcher {
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
           fallback_ctas = 4LL * sms;
       }
-      coarse_cap = (n > 3 && L > 2) ? coarse_cap_for(tile_coarse) : 0;
+      if (rgb) down_cap = down_cap_for(tile_down);
+      coarse_cap = ((n > 3 || rgb) && L > 2) ? coarse_cap_for(tile_coarse) : (rgb ? n : 0);
       coarse_smem = coarse_smem_for(tile_coarse);
       b5 = p.filter == HMP_FILTER_BINOMIAL5 && L > 1;
       if (L > 1 && !b5 && !generic) {
@@ -444,8 +452,8 @@ struct hmp_stitcher {
       // With three or more images pyr_down keeps the level-0 pixels for pyr_fine (one load per slot
       // instead of a table lookup and a gather); with two it measured slower (the extra writes
       // lengthen pyr_down more than they shorten pyr_fine), so pyr_fine gathers again.
-      use_p0 = L > 1 && !b5 && n >= 3 && !generic;
-      fine_cap = (use_p0 && n > 3) ? fine_cap_for() : 0;
+      use_p0 = L > 1 && !b5 && n >= 3 && !generic && !rgb;
+      fine_cap = (use_p0 && n > 3) || rgb ? fine_cap_for() : 0;
       for (int k = 0; use_p0 && k < n; ++k) {
         const hmp::PlaneDev& P = slot_planes[k];
         if (P.w <= 0 || P.h <= 0) continue;
@@ -468,7 +476,8 @@ struct hmp_stitcher {
     }
     if (generic) launches = hmp::generic_launches(p.levels, p.canvas_plane_used);
     if (p.levels > 1 && !b5 && !generic && p.canvas_plane_used) {
-      const hmp_status cs = setup_copy_blocks();
+      if (!rgb) plan_copies(cps);
+      const hmp_status cs = setup_copy_blocks(cps);
       if (cs.code != HMP_OK) return cs;
     }
     if (p.canvas_plane_used && p.levels > 0 && !generic) {
@@ -512,14 +521,18 @@ struct hmp_stitcher {
 
   // Copy blocks: plans them (for both pyramid down-tile edges the tile setter allows) and uploads
   // the work lists, the pyramid-block map the resolve pass marks and the alpha flag.
-  hmp_status setup_copy_blocks() {
+  void plan_copies(hmp::CopyPlan (&cps)[2]) const {
     const hmp::Plan& p = plan;
+    if (p.levels < 2) return;
     const int align = 1 << (p.levels - 1);
-    hmp::CopyPlan cps[2];
     for (int i = 0; i < 2; ++i) {
       const int td = i == 0 ? 32 : 64;
-      if (td % align == 0) hmp::plan_copy_blocks(p, td, tile_coarse, cps[i]);
+      if (td % align == 0) hmp::plan_copy_blocks(p, td, std::max(32, align / 2), cps[i]);
     }
+  }
+
+  hmp_status setup_copy_blocks(const hmp::CopyPlan (&cps)[2]) {
+    const hmp::Plan& p = plan;
     const hmp::CopyPlan& c = cps[1].usable ? cps[1] : cps[0];
     if (!c.usable) return ok_status();
     cudaError_t e = upload_list(c.fine_list, &fine_list);
@@ -573,7 +586,7 @@ struct hmp_stitcher {
   // Kernels one process() launches in copy-block mode: the flag reset, the listed pyramid kernels,
   // the gather and the three gated fallbacks.
   int copy_launches() const {
-    return (n_down[tile_down == 64 ? 1 : 0] > 0) + (n_coarse > 0) + (n_fine > 0) + 1 + (copy_opaque ? 0 : 1);
+    return (n_down[tile_down == 64 ? 1 : 0] > 0) + (n_coarse > 0) + (n_fine > 0) + 1 + (copy_opaque || rgb ? 0 : 1);
   }
 
   // Compulsory bytes per process(): outside the write rect, 4 (table) + 1 (seam) + a source and
@@ -606,7 +619,7 @@ struct hmp_stitcher {
     if (!directory) return make_status(HMP_ERR_INVALID_VALUE, "directory is null");
     if (p.levels == 0)
       return make_status(HMP_ERR_INVALID_VALUE, "Soft-blend pyramid is only available when num_levels > 0");
-    if (p.rule != hmp::kRuleTwo || b5 || (generic && p.channels != 4))
+    if (p.rule != hmp::kRuleTwo || b5 || p.channels != 4)
       return make_status(HMP_ERR_NOT_SUPPORTED,
                          "the pyramid dump covers two-image stitchers of RGBA pixels with the box filter");
     if (!have_last) return make_status(HMP_ERR_INVALID_VALUE, "No Laplacian workspace is populated yet: call process() first");
@@ -824,8 +837,7 @@ struct hmp_stitcher {
     return S;
   }
 
-  // uchar3 / float4 / float3 pixels: the canvas outside the write rect, then the pyramid level by
-  // level, all on the caller's stream (hmp_generic.cu).
+  // float4 / float3 pixels: the canvas outside the write rect, then the pyramid level by level, all on the caller's stream (hmp_generic.cu).
   hmp_status process_generic(const hmp::SrcSet& S, const hmp_image* canvas, cudaStream_t s) {
     const hmp::Plan& p = plan;
     hmp::CanvasDev C;
@@ -848,7 +860,7 @@ struct hmp_stitcher {
         g.skip_x1 = p.write.x + p.write.w;
         g.skip_y1 = p.write.y + p.write.h;
       }
-      e = hmp::launch_generic_canvas(g, p.channels, p.pixel_float, p.canvas_opaque, s);
+      e = hmp::launch_generic_canvas(g, p.channels, p.canvas_opaque, s);
       if (e != cudaSuccess) return cuda_status(e, "canvas launch");
     }
     if (p.levels > 0) {
@@ -874,9 +886,105 @@ struct hmp_stitcher {
       a.wy1 = a.wy0 + p.write.h;
       a.cx_off = p.blend.x;
       a.cy_off = p.blend.y;
-      e = hmp::launch_generic_pyramid(a, p.channels, p.pixel_float, p.rule, p.batch, Rg, s);
+      e = hmp::launch_generic_pyramid(a, p.channels, p.rule, p.batch, Rg, s);
       if (e != cudaSuccess) return cuda_status(e, "pyramid launch");
     }
+    return ok_status();
+  }
+
+  // uchar3 pixels: the canvas gather beside the pyramid over the blocks near a seam, as for RGBA8
+  // frames, without checks (hmp_rgb.cu).
+  hmp_status process_rgb(const hmp::SrcSet& S, const hmp::CanvasDev& C, bool packed, cudaStream_t s) {
+    const hmp::Plan& p = plan;
+    const int di = tile_down == 64 ? 1 : 0;
+    const long long longest = std::max<long long>({n_down[di], n_coarse, n_fine});
+    const bool copy = copy_plan && copy_on && (n_fine == 0 || down_list[di] != nullptr) &&
+                      longest * p.batch < (1LL << 31) - 1;
+    const bool gather = p.canvas_plane_used &&
+                        (p.levels == 0 || copy || p.write.w < p.canvas_w || p.write.h < p.canvas_h);
+    hmp::GatherArgs ga{};
+    ga.S = S;
+    ga.P = packed ? canvas_raw : canvas_plane;
+    ga.C = C;
+    ga.batch = p.batch;
+    ga.n_owners = p.n;
+    ga.seg_owner = seg_owner;
+    ga.seg_pitch = seg_pitch;
+    if (p.levels > 0 && !copy) {
+      ga.skip_x0 = p.write.x;
+      ga.skip_y0 = p.write.y;
+      ga.skip_x1 = p.write.x + p.write.w;
+      ga.skip_y1 = p.write.y + p.write.h;
+    }
+    const hmp::SkipMap blocks = copy ? skip : hmp::SkipMap{};
+    cudaError_t e = cudaSuccess;
+    if (p.levels == 0) {
+      tbegin(0, s);
+      e = hmp::launch_rgb_gather(ga, packed, blocks, s);
+      tend(0, s);
+      if (timing && tnext < kTimingSlots) ++tnext;
+      return e == cudaSuccess ? ok_status() : cuda_status(e, "canvas_gather launch");
+    }
+    const bool fork = gather && !serialize;
+    const cudaStream_t ps = fork ? aux : s;
+    if (fork) {
+      e = cudaEventRecord(ev_fork, s);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(aux, ev_fork, 0);
+      if (e != cudaSuccess) return cuda_status(e, "stream fork");
+    }
+    const char* what = "";
+    hmp::PyrArgs a = pyr_args(S, C);
+    a.R1 = R1;
+    a.list_frames = p.batch;
+    const auto grid_of = [&](const uint32_t* list, int n_list, dim3 dense) {
+      a.tiles = copy ? list : nullptr;
+      return copy ? dim3(unsigned(n_list) * unsigned(p.batch), 1, 1) : dense;
+    };
+    if (p.levels > 1 && (!copy || n_fine > 0)) {
+      dim3 g = grid_of(down_list[di], n_down[di],
+                       dim3((p.lw[0] + tile_down - 1) / tile_down, (p.lh[0] + tile_down - 1) / tile_down, p.batch));
+      a.tile = tile_down;
+      what = "pyr_down launch";
+      tbegin(1, ps);
+      e = hmp::launch_rgb_down(a, g, ps);
+      tend(1, ps);
+      if (e == cudaSuccess) {
+        const int x1hi = std::min(((a.wx1 - 1) >> 1) + 2, p.lw[1]), y1hi = std::min(((a.wy1 - 1) >> 1) + 2, p.lh[1]);
+        a.tile = tile_coarse;
+        a.tx0 = (a.wx0 >> 1) / tile_coarse;
+        a.ty0 = (a.wy0 >> 1) / tile_coarse;
+        g = grid_of(coarse_list, n_coarse, dim3((x1hi + tile_coarse - 1) / tile_coarse - a.tx0,
+                                                (y1hi + tile_coarse - 1) / tile_coarse - a.ty0, p.batch));
+        what = "pyr_coarse launch";
+        tbegin(2, ps);
+        e = hmp::launch_rgb_coarse(a, p.rule, g, coarse_smem, ps);
+        tend(2, ps);
+      }
+    }
+    if (e == cudaSuccess && (!copy || n_fine > 0)) {
+      const dim3 g = grid_of(fine_list, n_fine,
+                             dim3((a.wx1 - (a.wx0 & ~1) + 63) / 64, (a.wy1 - (a.wy0 & ~1) + 15) / 16, p.batch));
+      what = "pyr_fine launch";
+      tbegin(3, ps);
+      e = hmp::launch_rgb_fine(a, p.rule, g, ps);
+      tend(3, ps);
+    }
+    if (e == cudaSuccess && gather) {
+      what = "canvas_gather launch";
+      tbegin(0, s);
+      e = hmp::launch_rgb_gather(ga, packed, blocks, s);
+      tend(0, s);
+    }
+    if (fork) {  // also after a failed launch, so that the caller's stream waits for what was queued
+      const cudaError_t r = cudaEventRecord(ev_join, aux);
+      const cudaError_t w = cudaStreamWaitEvent(s, ev_join, 0);
+      if (e == cudaSuccess) {
+        e = r != cudaSuccess ? r : w;
+        what = "stream join";
+      }
+    }
+    if (e != cudaSuccess) return cuda_status(e, what);
+    if (timing && tnext < kTimingSlots) ++tnext;
     return ok_status();
   }
 
@@ -884,7 +992,7 @@ struct hmp_stitcher {
     const hmp::Plan& p = plan;
     if (!inputs || n_inputs != p.n) return make_status(HMP_ERR_INVALID_VALUE, "inputs size != N");
     if (!canvas || !canvas->data) return make_status(HMP_ERR_INVALID_DEVICE_POINTER, "Canvas must be provided");
-    const size_t pxb = size_t(p.pixel_bytes()), align = p.pixel_float ? 4 : (generic ? 1 : 4);
+    const size_t pxb = size_t(p.pixel_bytes()), align = rgb ? 1 : 4;
     if (canvas->width != p.canvas_w || canvas->height != p.canvas_h || canvas->pitch < size_t(canvas->width) * pxb ||
         canvas->pitch % align != 0)
       return make_status(HMP_ERR_INVALID_VALUE, "canvas size does not match the stitcher");
@@ -897,7 +1005,7 @@ struct hmp_stitcher {
       if (im.width <= 0 || im.height <= 0 || im.pitch < size_t(im.width) * pxb || im.pitch > size_t(INT_MAX) ||
           im.pitch % align != 0 || reinterpret_cast<uintptr_t>(im.data) % align != 0)
         return make_status(HMP_ERR_INVALID_VALUE, "input image has an invalid size, pitch or alignment");
-      if (!generic && size_t(im.height) * (im.pitch / 4) >= size_t(hmp::kOffMask) - 1)
+      if (!generic && !rgb && size_t(im.height) * (im.pitch / 4) >= size_t(hmp::kOffMask) - 1)
         return make_status(HMP_ERR_NOT_SUPPORTED, "input frames must hold fewer than 2^29 - 2 pixels");
       if (im.width >= 65535 || im.height >= 65535)
         return make_status(HMP_ERR_INVALID_VALUE, "input images must be smaller than 65535 pixels per side");
@@ -910,7 +1018,11 @@ struct hmp_stitcher {
     last_src = S;
     have_last = true;
     if (generic) return process_generic(S, canvas, s);
-    if (p.canvas_plane_used) {
+    // RGB8 frames past the resolved offsets' range (byte offsets below 2^29 - 2) take the packed entries.
+    bool packed = false;
+    for (int i = 0; rgb && i < p.n; ++i)
+      packed = packed || size_t(S.h[i]) * size_t(S.pitch[i]) >= size_t(hmp::kOffMask) - 1;
+    if (p.canvas_plane_used && !packed) {
       // The gather reads the canvas plane as offsets into these frames: resolve it for their
       // geometry on the first call and whenever a size or pitch changes.
       bool same = resolved;
@@ -918,7 +1030,7 @@ struct hmp_stitcher {
         same = same && S.w[i] == geo_w[i] && S.h[i] == geo_h[i] && S.pitch[i] == geo_pitch[i];
       if (!same) {
         const cudaError_t re = hmp::launch_resolve_plane(canvas_raw, const_cast<uint32_t*>(canvas_plane.map), seg_owner,
-                                                         seg_pitch, S, p.n, p.canvas_opaque,
+                                                         seg_pitch, S, p.n, p.canvas_opaque && !rgb, rgb,
                                                          copy_plan ? skip : hmp::SkipMap{}, s);
         if (re != cudaSuccess) return cuda_status(re, "canvas plane resolve launch");
         for (int i = 0; i < p.n; ++i) {
@@ -935,6 +1047,7 @@ struct hmp_stitcher {
     C.bstride = (long long)canvas->pitch * canvas->height;
     C.w = canvas->width;
     C.h = canvas->height;
+    if (rgb) return process_rgb(S, C, packed, s);
 
     // Copy-block mode for this call: planned, switched on, and every table entry the copy blocks
     // read lies inside these frames (else it would read as a fill).
@@ -1276,7 +1389,7 @@ HMP_API hmp_status hmp_stitcher_set_tiles(hmp_stitcher* st, int tile_down, int t
     return make_status(HMP_ERR_INVALID_VALUE, "tile_down must be 32 or 64 and a multiple of 2^(levels-1)");
   if (tile_coarse != 32 || (tile_coarse * 2) % align != 0)
     return make_status(HMP_ERR_INVALID_VALUE, "tile_coarse must be 32");
-  const int cap = p.n > 3 ? st->down_cap_for(tile_down) : 0;
+  const int cap = p.n > 3 || st->rgb ? st->down_cap_for(tile_down) : 0;
   if (hmp::pyr_down_smem(cap > 0 ? cap : p.n, tile_down) > 227 * 1024)
     return make_status(HMP_ERR_NOT_SUPPORTED, "pyramid tile does not fit in shared memory");
   st->tile_down = tile_down;
