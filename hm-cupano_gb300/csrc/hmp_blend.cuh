@@ -147,9 +147,11 @@ __device__ __forceinline__ float4 blend_three(const float4* L, float m0, float m
       }
     return r;
   }
-  m0 /= sum;
-  m1 /= sum;
-  m2 /= sum;
+  if (sum != 1.f) {  // x / 1 is x
+    m0 /= sum;
+    m1 /= sum;
+    m2 /= sum;
+  }
   float aout = 0.f;
   if (m0 > 0.f && L[0].w > aout) aout = L[0].w;
   if (m1 > 0.f && L[1].w > aout) aout = L[1].w;
@@ -165,7 +167,7 @@ __device__ __forceinline__ float4 blend_nway(const float4* L, int n, float* w) {
 #pragma unroll
   for (int k = 0; k < NMAX; ++k)
     if (k < n) sumw += w[k];
-  if (sumw > 0.f) {
+  if (sumw > 0.f && sumw != 1.f) {
 #pragma unroll
     for (int k = 0; k < NMAX; ++k)
       if (k < n) w[k] /= sumw;
@@ -191,9 +193,11 @@ __device__ __forceinline__ float4 blend_nway(const float4* L, int n, float* w) {
       if (k == aidx && amax != 0.f) r = L[k];
     return r;
   }
+  if (sumw2 != 1.f) {
 #pragma unroll
-  for (int k = 0; k < NMAX; ++k)
-    if (k < n) w[k] /= sumw2;
+    for (int k = 0; k < NMAX; ++k)
+      if (k < n) w[k] /= sumw2;
+  }
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int k = 0; k < NMAX; ++k) {
@@ -342,7 +346,7 @@ __device__ __forceinline__ float4 nway_lap_blend(int n, int na, uint32_t list, u
   float sumw2 = 0.f;
   for (int c = 0; c < na; ++c) {
     float w = __ldg(mk + ((list >> (4 * c)) & 15u));
-    if (sumw > 0.f) w /= sumw;
+    if (sumw > 0.f && sumw != 1.f) w /= sumw;
     const float4 g = pix(c);
     if (g.w > amax) {
       amax = g.w;
@@ -356,10 +360,10 @@ __device__ __forceinline__ float4 nway_lap_blend(int n, int na, uint32_t list, u
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int c = 0; c < na; ++c) {
     float w = __ldg(mk + ((list >> (4 * c)) & 15u));
-    if (sumw > 0.f) w /= sumw;
+    if (sumw > 0.f && sumw != 1.f) w /= sumw;
     const float4 g = pix(c);
     if (g.w == 0.f) w = 0.f;
-    w /= sumw2;
+    if (sumw2 != 1.f) w /= sumw2;
     const float4 L = lap(c, g);
     acc.x += w * L.x;
     acc.y += w * L.y;

@@ -74,8 +74,23 @@ __device__ __forceinline__ const uchar4* slot_src(const PyrArgs& a, int k, int o
   return p;
 }
 
-__device__ __forceinline__ float4 u32_to_f4(uint32_t v) {
-  return make_float4(float(v & 0xFFu), float((v >> 8) & 0xFFu), float((v >> 16) & 0xFFu), float(v >> 24));
+// Alpha-aware mean of a 2x2 block of level-0 pixels (r0: the upper pair, r1: the lower; xin / yin: the
+// second column / row lies inside the level), as DownAcc's. Four opaque pixels, which camera frames
+// hold everywhere they are mapped, are summed as packed integers (sums below 2^10, exact).
+__device__ __forceinline__ float4 down0(uint2 r0, uint2 r1, bool xin, bool yin) {
+  if (xin && yin && (r0.x & r0.y & r1.x & r1.y) >= 0xFF000000u) {
+    const uint32_t rb = (r0.x & 0xFF00FFu) + (r0.y & 0xFF00FFu) + (r1.x & 0xFF00FFu) + (r1.y & 0xFF00FFu);
+    const uint32_t g = ((r0.x >> 8) & 0xFFu) + ((r0.y >> 8) & 0xFFu) + ((r1.x >> 8) & 0xFFu) + ((r1.y >> 8) & 0xFFu);
+    return make_float4((__uint_as_float(0x4B000000u | (rb & 0xFFFFu)) - 8388608.0f) * 0.25f,
+                       (__uint_as_float(0x4B000000u | g) - 8388608.0f) * 0.25f,
+                       (__uint_as_float(0x4B000000u | (rb >> 16)) - 8388608.0f) * 0.25f, 255.f);
+  }
+  DownAcc acc;
+  acc.add(u32_to_f4(r0.x));
+  if (xin) acc.add(u32_to_f4(r0.y));
+  if (yin) acc.add(u32_to_f4(r1.x));
+  if (xin && yin) acc.add(u32_to_f4(r1.y));
+  return acc.result();
 }
 
 // Level-l buffer of slot k, frame b (k selected at run time among the NMAX slots).
@@ -89,10 +104,7 @@ __device__ __forceinline__ Store* level_of(const PyrArgs& a, int k, int l, int b
 }
 
 // Gaussian levels 1..L-1 of every slot for one TD x TD level-0 tile (TD a multiple of 2^(L-1),
-// so no level needs a neighbouring tile). Level 0 is gathered like the canvas: each warp owns
-// tile rows, copies their table entries into shared memory (cp.async, 32 consecutive entries
-// per instruction), then replaces every entry by its source pixel (one 4-byte cp.async each, all
-// in flight together). One pass then reduces each 4x4 pixel block to its four level-1 pixels
+// so no level needs a neighbouring tile). Level 0 is gathered into shared memory (gather_slot). One pass then reduces each 4x4 pixel block to its four level-1 pixels
 // (kept in registers and stored to HBM) and their level-2 pixel; deeper levels reduce the
 // previous level in shared memory (levels 3, 5 reuse the level-0 buffer). Every level >= 1 goes
 // to HBM. A slot whose plane misses the tile produces zeros, which its level buffers already
@@ -184,6 +196,89 @@ __device__ __forceinline__ bool support_alpha_zero(const PyrArgs& a, int x, int 
   return (v >> 24) == 0u && __ldg(a.support_mark + (long long)(y >> a.sm_shift) * a.sm_pitch + (x >> a.sm_shift)) != 0;
 }
 
+// Source pixel address of slot k (k and the owner known only at run time), as slot_src.
+__device__ __forceinline__ const uchar4* slot_src_dyn(const PyrArgs& a, int k, int o, uint32_t e, int b, bool opaque,
+                                                      uint32_t& fill) {
+  const int sx = int(e & 0xFFFFu), sy = int(e >> 16);
+  fill = 0u;
+  if (a.slot[k].owner == nullptr) o = k;
+  if (o >= kDevMaxImages) return nullptr;
+  if (sx < a.S.w[o] && sy < a.S.h[o])
+    return reinterpret_cast<const uchar4*>(reinterpret_cast<const char*>(a.S.ptr[o]) + b * a.S.bstride[o] +
+                                           (long long)sy * int(a.S.pitch[o])) + sx;
+  if (opaque && sx != 0xFFFF) fill = 0xFF000000u;
+  return nullptr;
+}
+
+// Level 0 of slot k over a TD x TD tile, into pk (0 outside the plane): a warp takes every eighth
+// row, its lanes 32 consecutive pixels; the table entries of kBatch pixels are loaded together, then
+// their source pixels. A slot of one image has its frame's base, size and pitch in registers, so a
+// pixel costs a compare and a multiply-add besides its loads. keep: also stored for pyr_fine.
+// Before (entries and pixels through cp.async, the frame looked up per pixel) the kernels spent their
+// issue slots on addresses: eight images 9000x2400, 1663 tiles, 64.4 -> 52.5 us; three 6000x1800 FP16,
+// 855 tiles, 32.8 -> 31.2; two 8500x3300, 318 tiles, 18.6 -> 17.2 (alone, cold).
+template <int TD>
+__device__ __forceinline__ void gather_slot(const PyrArgs& a, int k, uint32_t* pk, int X0, int Y0, int b, bool opaque,
+                                            bool keep) {
+  constexpr int NJ = TD / 32, ROWS = TD / 8, kBatch = 8, kSteps = ROWS * NJ;
+  static_assert(kSteps % kBatch == 0 || kSteps < kBatch, "whole batches");
+  constexpr int N = kSteps < kBatch ? kSteps : kBatch;
+  const PlaneDev& P = a.slot[k];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x1 = min(P.x0 + P.w, a.lw[0]), y1 = min(P.y0 + P.h, a.lh[0]);
+  const long long mrow = 8LL * P.map_pitch;
+  const uint32_t* m = P.map + (long long)(Y0 + warp - P.y0) * P.map_pitch + (X0 + lane - P.x0);
+  bool cin[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) cin[j] = X0 + lane + 32 * j >= P.x0 && X0 + lane + 32 * j < x1;
+#pragma unroll
+  for (int g = 0; g < kSteps; g += N) {
+    uint32_t e[N], v[N];
+    unsigned in = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int i = (g + u) / NJ, j = (g + u) % NJ, y = Y0 + warp + 8 * i;
+      const bool t = cin[j] && y >= P.y0 && y < y1;
+      e[u] = t ? __ldg(m + i * mrow + 32 * j) : 0xFFFFFFFFu;
+      if (t) in |= 1u << u;
+    }
+    if (P.owner == nullptr) {
+      const char* base = reinterpret_cast<const char*>(a.S.ptr[k]) + b * a.S.bstride[k];
+      const int fw = a.S.w[k], fh = a.S.h[k], pitch = int(a.S.pitch[k]);
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const int sx = int(e[u] & 0xFFFFu), sy = int(e[u] >> 16);
+        v[u] = opaque && sx != 0xFFFF ? 0xFF000000u : 0u;
+        if (sx < fw && sy < fh) v[u] = __ldg(reinterpret_cast<const uint32_t*>(base + (long long)sy * pitch) + sx);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const int i = (g + u) / NJ, j = (g + u) % NJ;
+        int o = 0xFF;
+        if ((in >> u) & 1u)
+          o = int(__ldg(P.owner + (long long)(Y0 + warp + 8 * i - P.y0) * P.owner_pitch + (X0 + lane + 32 * j - P.x0)));
+        uint32_t fill;
+        const uchar4* sp = slot_src_dyn(a, k, o, e[u], b, opaque, fill);
+        v[u] = sp ? __ldg(reinterpret_cast<const uint32_t*>(sp)) : fill;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int i = (g + u) / NJ, j = (g + u) % NJ;
+      pk[(warp + 8 * i) * TD + lane + 32 * j] = v[u];
+    }
+    if (keep) {
+      uint32_t* d = a.P0[k] + (long long)b * P.w * P.h + (long long)(Y0 + warp - P.y0) * P.w + (X0 + lane - P.x0);
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const int i = (g + u) / NJ, j = (g + u) % NJ;
+        if ((in >> u) & 1u) d[(long long)(8 * i) * P.w + 32 * j] = v[u];
+      }
+    }
+  }
+}
+
 // kListed: work lists and the fallback gate (copy-block mode); always on for three or more images,
 // a separate instantiation for two, whose dense kernels stay free of that code.
 template <int NMAX, typename Store, int TD, bool kListed = false, bool kWalk = false>
@@ -203,7 +298,7 @@ __global__ void __launch_bounds__(256) pyr_down_kernel(const __grid_constant__ P
     uint32_t* pix = reinterpret_cast<uint32_t*>(sm);  // level 0: [n][TD][TD] pixels
     float4* bufA = sm;                                // levels 3, 5: [n][T1*T1], over level 0
     float4* bufB = sm + n * T1 * T1;                  // levels 2, 4, 6: [n][T2*T2]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int X0 = tx * TD, Y0 = ty * TD;
     const bool opaque = a.opaque != 0;
     const int L = a.levels;
@@ -216,75 +311,13 @@ __global__ void __launch_bounds__(256) pyr_down_kernel(const __grid_constant__ P
       active[k] = k < n && !(X0 >= P.x0 + P.w || Y0 >= P.y0 + P.h || X0 + TD <= P.x0 || Y0 + TD <= P.y0);
       if (active[k]) amask |= 1u << k;
     }
-    // Level 0, step 1: table entries (the sentinel outside the level or the plane).
+    // Level 0; with three and more images also kept for pyr_fine inside the slot's plane, so that the
+    // level-0 pass reads the pixels back instead of repeating the table lookups and gathers.
+    const bool keep = kKeepLevel0 && a.use_p0 && keeps_level0<(NMAX >= 3 || kListed), kWalk>(a);
   #pragma unroll
-    for (int k = 0; k < NMAX; ++k) {
-      if (!active[k]) continue;
-      const PlaneDev& P = a.slot[k];
-      uint32_t* pk = pix + k * TD * TD;
-      for (int r = warp; r < TD; r += 8) {
-        const int y = Y0 + r, ry = y - P.y0;
-  #pragma unroll
-        for (int j = 0; j < TD / 32; ++j) {
-          const int x = X0 + 32 * j + lane, rx = x - P.x0;
-          uint32_t* d = pk + r * TD + 32 * j + lane;
-          if (x < lw0 && y < lh0 && (unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-            cp_async<4>(d, P.map + (long long)ry * P.map_pitch + rx);
-          else
-            *d = 0xFFFFFFFFu;
-        }
-      }
-    }
-    cp_async_commit_wait_all();
-    // Step 2: each thread replaces the entries it copied by their source pixels.
-  #pragma unroll
-    for (int k = 0; k < NMAX; ++k) {
-      if (!active[k]) continue;
-      const PlaneDev& P = a.slot[k];
-      uint32_t* pk = pix + k * TD * TD;
-      for (int r = warp; r < TD; r += 8) {
-        const int y = Y0 + r, ry = y - P.y0;
-  #pragma unroll
-        for (int j = 0; j < TD / 32; ++j) {
-          const int x = X0 + 32 * j + lane, rx = x - P.x0;
-          uint32_t* d = pk + r * TD + 32 * j + lane;
-          const uint32_t e = *d;
-          int o = k;
-          if (P.owner != nullptr)
-            o = (x < lw0 && y < lh0 && (unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-                    ? int(__ldg(P.owner + (long long)ry * P.owner_pitch + rx))
-                    : 0xFF;
-          uint32_t fill;
-          const uchar4* sp = slot_src<NMAX>(a, k, o, e, b, opaque, fill);
-          if (sp)
-            cp_async<4>(d, sp);
-          else
-            *d = fill;
-        }
-      }
-    }
-    cp_async_commit_wait_all();
+    for (int k = 0; k < NMAX; ++k)
+      if (active[k]) gather_slot<TD>(a, k, pix + k * TD * TD, X0, Y0, b, opaque, keep);
     __syncthreads();
-    // Level 0 for pyr_fine: each slot's gathered pixels inside its plane rect, so that the level-0
-    // pass reads them back directly instead of repeating the table lookups and gathers.
-    if constexpr (kKeepLevel0) {
-  #pragma unroll
-      for (int k = 0; k < NMAX; ++k) {
-        if (!active[k] || !a.use_p0 || !keeps_level0<(NMAX >= 3 || kListed), kWalk>(a)) continue;
-        const PlaneDev& P = a.slot[k];
-        uint32_t* dst = a.P0[k] + (long long)b * P.w * P.h;
-        const uint32_t* pk = pix + k * TD * TD;
-        for (int r = warp; r < TD; r += 8) {
-          const int ry = Y0 + r - P.y0;
-          if ((unsigned)ry >= (unsigned)P.h) continue;
-  #pragma unroll
-          for (int j = 0; j < TD / 32; ++j) {
-            const int x = X0 + 32 * j + lane, rx = x - P.x0;
-            if ((unsigned)rx < (unsigned)P.w) dst[(long long)ry * P.w + rx] = pk[r * TD + 32 * j + lane];
-          }
-        }
-      }
-    }
     // Levels 1 and 2: one item = one level-2 pixel of one slot = its four level-1 pixels, each the
     // alpha-aware mean of a 2x2 level-0 block (two 8-byte shared loads), summed in (0,0), (1,0),
     // (0,1), (1,1) order at both levels.
@@ -305,13 +338,7 @@ __global__ void __launch_bounds__(256) pyr_down_kernel(const __grid_constant__ P
         if (gx < lw1 && gy < lh1) {
           const uint2 r0 = *reinterpret_cast<const uint2*>(pk + (2 * ty) * TD + 2 * tx);
           const uint2 r1 = *reinterpret_cast<const uint2*>(pk + (2 * ty + 1) * TD + 2 * tx);
-          const bool xin = 2 * gx + 1 < lw0, yin = 2 * gy + 1 < lh0;
-          DownAcc acc;
-          acc.add(u32_to_f4(r0.x));
-          if (xin) acc.add(u32_to_f4(r0.y));
-          if (yin) acc.add(u32_to_f4(r1.x));
-          if (xin && yin) acc.add(u32_to_f4(r1.y));
-          const float4 v = acc.result();
+          const float4 v = down0(r0, r1, 2 * gx + 1 < lw0, 2 * gy + 1 < lh0);
           store_level(G1 + (long long)gy * lw1 + gx, v);
           acc2.add(v);
         }
@@ -364,20 +391,6 @@ __global__ void __launch_bounds__(256) pyr_down_kernel(const __grid_constant__ P
   }
 }
 
-// Source pixel address of slot k (k and the owner known only at run time), as slot_src.
-__device__ __forceinline__ const uchar4* slot_src_dyn(const PyrArgs& a, int k, int o, uint32_t e, int b, bool opaque,
-                                                      uint32_t& fill) {
-  const int sx = int(e & 0xFFFFu), sy = int(e >> 16);
-  fill = 0u;
-  if (a.slot[k].owner == nullptr) o = k;
-  if (o >= kDevMaxImages) return nullptr;
-  if (sx < a.S.w[o] && sy < a.S.h[o])
-    return reinterpret_cast<const uchar4*>(reinterpret_cast<const char*>(a.S.ptr[o]) + b * a.S.bstride[o] +
-                                           (long long)sy * int(a.S.pitch[o])) + sx;
-  if (opaque && sx != 0xFFFF) fill = 0xFF000000u;
-  return nullptr;
-}
-
 // pyr_down for the N-way rule (up to eight slots). A tile of the N-image blend region overlaps
 // only one to three slots' planes, so instead of loops unrolled over all eight slots (whose code
 // and per-slot checks dominated: instruction-cache stalls) the tile's active slots form a run-time
@@ -397,7 +410,7 @@ __global__ void __launch_bounds__(256) pyr_down_n_kernel(const __grid_constant__
     uint32_t* pix = reinterpret_cast<uint32_t*>(sm);  // level 0: [cap][TD][TD]
     float4* bufA = sm;                                // levels 3, 5: [cap][T1*T1], over level 0
     float4* bufB = sm + cap * T1 * T1;                // levels 2, 4, 6: [cap][T2*T2]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int X0 = tx * TD, Y0 = ty * TD;
     const bool opaque = a.opaque != 0;
     const int L = a.levels;
@@ -409,70 +422,11 @@ __global__ void __launch_bounds__(256) pyr_down_n_kernel(const __grid_constant__
       if (!(X0 >= P.x0 + P.w || Y0 >= P.y0 + P.h || X0 + TD <= P.x0 || Y0 + TD <= P.y0) && na < cap)
         list |= uint32_t(k) << (4 * na++);
     }
+    const bool keep = a.use_p0 && keeps_level0<true, kWalk>(a);
   #pragma unroll 1
-    for (int c = 0; c < na; ++c) {
-      const PlaneDev& P = a.slot[(list >> (4 * c)) & 15u];
-      uint32_t* pk = pix + c * TD * TD;
-      for (int r = warp; r < TD; r += 8) {
-        const int y = Y0 + r, ry = y - P.y0;
-  #pragma unroll
-        for (int j = 0; j < TD / 32; ++j) {
-          const int x = X0 + 32 * j + lane, rx = x - P.x0;
-          uint32_t* d = pk + r * TD + 32 * j + lane;
-          if (x < lw0 && y < lh0 && (unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-            cp_async<4>(d, P.map + (long long)ry * P.map_pitch + rx);
-          else
-            *d = 0xFFFFFFFFu;
-        }
-      }
-    }
-    cp_async_commit_wait_all();
-  #pragma unroll 1
-    for (int c = 0; c < na; ++c) {
-      const int k = (list >> (4 * c)) & 15u;
-      const PlaneDev& P = a.slot[k];
-      uint32_t* pk = pix + c * TD * TD;
-      for (int r = warp; r < TD; r += 8) {
-        const int y = Y0 + r, ry = y - P.y0;
-  #pragma unroll
-        for (int j = 0; j < TD / 32; ++j) {
-          const int x = X0 + 32 * j + lane, rx = x - P.x0;
-          uint32_t* d = pk + r * TD + 32 * j + lane;
-          const uint32_t e = *d;
-          int o = k;
-          if (P.owner != nullptr)
-            o = (x < lw0 && y < lh0 && (unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-                    ? int(__ldg(P.owner + (long long)ry * P.owner_pitch + rx))
-                    : 0xFF;
-          uint32_t fill;
-          const uchar4* sp = slot_src_dyn(a, k, o, e, b, opaque, fill);
-          if (sp)
-            cp_async<4>(d, sp);
-          else
-            *d = fill;
-        }
-      }
-    }
-    cp_async_commit_wait_all();
+    for (int c = 0; c < na; ++c)
+      gather_slot<TD>(a, (list >> (4 * c)) & 15u, pix + c * TD * TD, X0, Y0, b, opaque, keep);
     __syncthreads();
-    if (a.use_p0 && keeps_level0<true, kWalk>(a)) {
-  #pragma unroll 1
-      for (int c = 0; c < na; ++c) {
-        const int k = (list >> (4 * c)) & 15u;
-        const PlaneDev& P = a.slot[k];
-        uint32_t* dst = a.P0[k] + (long long)b * P.w * P.h;
-        const uint32_t* pk = pix + c * TD * TD;
-        for (int r = warp; r < TD; r += 8) {
-          const int ry = Y0 + r - P.y0;
-          if ((unsigned)ry >= (unsigned)P.h) continue;
-  #pragma unroll
-          for (int j = 0; j < TD / 32; ++j) {
-            const int x = X0 + 32 * j + lane, rx = x - P.x0;
-            if ((unsigned)rx < (unsigned)P.w) dst[(long long)ry * P.w + rx] = pk[r * TD + 32 * j + lane];
-          }
-        }
-      }
-    }
     const bool has2 = L > 2;
     const int lw2 = a.lw[has2 ? 2 : 1], lh2 = a.lh[has2 ? 2 : 1];
   #pragma unroll 1
@@ -491,13 +445,7 @@ __global__ void __launch_bounds__(256) pyr_down_n_kernel(const __grid_constant__
         if (gx < lw1 && gy < lh1) {
           const uint2 r0 = *reinterpret_cast<const uint2*>(pk + (2 * ty) * TD + 2 * tx);
           const uint2 r1 = *reinterpret_cast<const uint2*>(pk + (2 * ty + 1) * TD + 2 * tx);
-          const bool xin = 2 * gx + 1 < lw0, yin = 2 * gy + 1 < lh0;
-          DownAcc acc;
-          acc.add(u32_to_f4(r0.x));
-          if (xin) acc.add(u32_to_f4(r0.y));
-          if (yin) acc.add(u32_to_f4(r1.x));
-          if (xin && yin) acc.add(u32_to_f4(r1.y));
-          const float4 v = acc.result();
+          const float4 v = down0(r0, r1, 2 * gx + 1 < lw0, 2 * gy + 1 < lh0);
           store_level(G1 + (long long)gy * lw1 + gx, v);
           acc2.add(v);
         }
@@ -1014,6 +962,25 @@ __device__ __forceinline__ float3 up_tile(const T* t, int i, bool ox, bool oy) {
   return make_float3(0.f, 0.f, 0.f);
 }
 
+// up_tile where every tap has alpha: the same bits without the tests.
+template <typename T>
+__device__ __forceinline__ float3 up_tile_solid(const T* t, int i, bool ox, bool oy) {
+  const float4 p = load_level(t + i);
+  if (!ox && !oy) return make_float3(p.x, p.y, p.z);
+  if (ox != oy) {
+    const float4 q = load_level(t + i + (ox ? 1 : kFineTW));
+    return make_float3(p.x * 0.5f + q.x * 0.5f, p.y * 0.5f + q.y * 0.5f, p.z * 0.5f + q.z * 0.5f);
+  }
+  const float4 q = load_level(t + i + 1), r = load_level(t + i + kFineTW), s = load_level(t + i + kFineTW + 1);
+  return make_float3(((p.x * 0.25f + q.x * 0.25f) + r.x * 0.25f) + s.x * 0.25f,
+                     ((p.y * 0.25f + q.y * 0.25f) + r.y * 0.25f) + s.y * 0.25f,
+                     ((p.z * 0.25f + q.z * 0.25f) + r.z * 0.25f) + s.z * 0.25f);
+}
+template <typename T>
+__device__ __forceinline__ float3 up_tile_either(bool solid, const T* t, int i, bool ox, bool oy) {
+  return solid ? up_tile_solid(t, i, ox, oy) : up_tile(t, i, ox, oy);
+}
+
 // pyr_fine: level 0 of the write region. A CTA owns a 64 x 16 pixel block, each warp 64 x 2 of
 // it, each lane the 2x2 quad (X, Y)..(X+1, Y+1). The CTA first copies its level-1 tiles (G^1 of
 // every slot, R^1) into shared memory with cp.async, then issues all its table lookups and
@@ -1057,6 +1024,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
     // arrays would not fit in registers four times over.
     constexpr int QB = NMAX > 3 ? 1 : 4;
     const int ti = warp * kFineTW + lane;  // tap (0,0) of the quad in the tiles
+    bool solid = false;  // every tap of the tiles has alpha
   #pragma unroll
     for (int q0 = 0; q0 < 4; q0 += QB) {
       int own[QB][NMAX], mv[QB];
@@ -1116,7 +1084,14 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
         }
       if (q0 == 0 && has1) {
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();
+        bool mine = true;  // a thread's own copies
+        for (int j = tid; j < kFineTA; j += 256) {
+          mine = mine && rs[j].w != 0.f;
+  #pragma unroll
+          for (int k = 0; k < NMAX; ++k)
+            if ((amask >> k) & 1u) mine = mine && load_level(gs + k * kFineTA + j).w != 0.f;
+        }
+        solid = __syncthreads_and(mine);
       }
       bool bad = false;  // copy-block mode: alpha 0 of the label image inside a copy block's support
   #pragma unroll
@@ -1150,7 +1125,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
             if (k == pk) sp = src[u][k];
           float4 g = to_f4(sp);
           if (has1 && ((amask >> pk) & 1u)) {  // an inactive slot's G^1 taps are all zero here
-            const float3 up = up_tile(gs + pk * kFineTA, ti, ox, oy);
+            const float3 up = up_tile_either(solid, gs + pk * kFineTA, ti, ox, oy);
             g.x = g.x - up.x;
             g.y = g.y - up.y;
             g.z = g.z - up.z;
@@ -1162,7 +1137,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
           for (int k = 0; k < NMAX; ++k) {
             float4 g = to_f4(src[u][k]);
             if (has1 && ((amask >> k) & 1u)) {
-              const float3 up = up_tile(gs + k * kFineTA, ti, ox, oy);
+              const float3 up = up_tile_either(solid, gs + k * kFineTA, ti, ox, oy);
               g.x = g.x - up.x;
               g.y = g.y - up.y;
               g.z = g.z - up.z;
@@ -1172,7 +1147,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
           r = blend_level0<RULE, NMAX>(n, lap, mv[u]);
         }
         if (has1) {
-          const float3 up = up_tile(rs, ti, ox, oy);
+          const float3 up = up_tile_either(solid, rs, ti, ox, oy);
           r.x = up.x + r.x;
           r.y = up.y + r.y;
           r.z = up.z + r.z;
@@ -1296,7 +1271,12 @@ __global__ void __launch_bounds__(256) pyr_fine_n_kernel(const __grid_constant__
       }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
+    bool mine = true;  // every tap this thread copied has alpha
+    for (int j = tid; j < kFineTA; j += 256) {
+      mine = mine && rs[j].w != 0.f;
+      for (int c = 0; c < na; ++c) mine = mine && load_level(gs + c * kFineTA + j).w != 0.f;
+    }
+    const bool solid = __syncthreads_and(mine);
   #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (!live[q]) continue;
@@ -1305,11 +1285,11 @@ __global__ void __launch_bounds__(256) pyr_fine_n_kernel(const __grid_constant__
       float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
       if (pc[q] >= 0) {
         const uint32_t g = pp[q];
-        const float3 up = up_tile(gs + pc[q] * kFineTA, ti, ox, oy);
-        r = make_float4(float(g & 0xFF) - up.x, float((g >> 8) & 0xFF) - up.y, float((g >> 16) & 0xFF) - up.z,
-                        float(g >> 24));
+        const float3 up = up_tile_either(solid, gs + pc[q] * kFineTA, ti, ox, oy);
+        const float4 f = u32_to_f4(g);
+        r = make_float4(f.x - up.x, f.y - up.y, f.z - up.z, f.w);
       }
-      const float3 up = up_tile(rs, ti, ox, oy);
+      const float3 up = up_tile_either(solid, rs, ti, ox, oy);
       r.x = up.x + r.x;
       r.y = up.y + r.y;
       r.z = up.z + r.z;

@@ -81,14 +81,6 @@ __device__ __forceinline__ RgbAt rgb_find(const SrcSet& S, int n, int o, uint32_
   return rgb_at(rgb_frame(S, o, b), (long long)sy * S.pitch[o] + 3LL * sx);
 }
 
-// Bytes of a word as floats: the byte in the low bits of 2^23, less 2^23 (a conversion costs four of
-// these).
-__device__ __forceinline__ float3 rgb_f3(uint32_t v) {
-  return make_float3(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440)) - 8388608.0f,
-                     __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7441)) - 8388608.0f,
-                     __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7442)) - 8388608.0f);
-}
-
 // Tile (tx, ty) and frame b of this CTA: the dense grid, or entry blockIdx.x of the work list, the
 // frames of a call fastest.
 __device__ __forceinline__ void rgb_tile(const PyrArgs& a, int& tx, int& ty, int& b) {
@@ -567,7 +559,8 @@ __global__ void __launch_bounds__(256) rgb_fine_kernel(const __grid_constant__ P
     if (!live[q]) continue;
     const bool ox = (q & 1) != 0, oy = (q >> 1) != 0;
     const auto lap = [&](int k, uint32_t p) {
-      float3 r = rgb_f3(p);
+      const float4 f = u32_to_f4(p);
+      float3 r = make_float3(f.x, f.y, f.z);
       const uint32_t c = (cmap >> (4 * k)) & 15u;
       if (has1 && c < 15u) {
         const float3 u = rgb_up(gs + c * kFineTA, ti, 1, kFineTW, ox, oy);
