@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from dataclasses import dataclass, field
 from typing import Iterable, Sequence
 
@@ -424,6 +425,68 @@ def _image(t) -> Image:
     return Image(C.c_void_p(t.data_ptr()), int(W), int(H), int(pitch) * t.element_size())
 
 
+# hmp_image records as native-aligned bytes (data, width, height, pitch), packed per call: a frame's
+# host cost is mostly this marshalling, and one pack costs what filling one ctypes field does.
+_PACK_IMAGES = {n: struct.Struct("@" + "PiiN" * n).pack for n in range(1, 10)}
+
+
+def _pack_images(tensors, batch: int, pixel: tuple | None = None):
+    """(packed hmp_image records, channels, float samples, device index) of tensors that all pass
+    _image's checks, share one pixel type (`pixel` if given), hold `batch` frames each and live on
+    one CUDA device; None otherwise, and the caller's checked path says why (or takes the call)."""
+    import torch
+
+    if len(tensors) not in _PACK_IMAGES:
+        return None
+    fields = []
+    dev = dtype = ch = None
+    for t in tensors:
+        if type(t) is not torch.Tensor or not t.is_cuda:
+            return None
+        shape, strides = t.shape, t.stride()
+        if len(shape) == 4:
+            b, h, w, c = shape
+            sb, sh, sw, sc = strides
+        elif len(shape) == 3:
+            h, w, c = shape
+            sh, sw, sc = strides
+            b, sb = 1, 0
+        else:
+            return None
+        if ch is None:
+            ch, dtype, dev = c, t.dtype, t.get_device()
+            if c not in (3, 4) or dtype not in (torch.uint8, torch.float32):
+                return None
+        elif c != ch or t.dtype != dtype or t.get_device() != dev:
+            return None
+        pitch = sh if h > 1 else w * c
+        if b != batch or sc != 1 or (w > 1 and sw != c) or pitch < w * c or (b > 1 and sb != pitch * h):
+            return None
+        fields += (t.data_ptr(), w, h, pitch if dtype is torch.uint8 else 4 * pitch)
+    if pixel is not None and (ch, dtype is torch.float32) != pixel:
+        return None
+    return _PACK_IMAGES[len(tensors)](*fields), ch, dtype is torch.float32, dev
+
+
+def _raw(name: str):
+    """A library function that takes packed images (bytes) where its declared form takes pointers."""
+    fn = _RAW.get(name)
+    if fn is None:
+        fn = _lib.lib()[name]
+        args, fn.restype = _lib.SIGNATURES[name]
+        fn.argtypes = [C.c_void_p if issubclass(a, C._Pointer) else a for a in args]
+        _RAW[name] = fn
+    return fn
+
+
+_RAW: dict = {}
+
+
+def _current_stream(torch, device: int) -> int:
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # what current_stream() wraps
+    return raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream
+
+
 class _Stitcher:
     _kind = 0
 
@@ -550,6 +613,32 @@ class _Stitcher:
         return {names[i]: (float(t.total_ms[i]), int(t.launches[i])) for i in range(4)}
 
     def _run(self, inputs: Sequence, canvas=None, stream=None):
+        """One process() call. Calls that pass every check go straight to the library, which returns
+        the sticky status itself; any other takes the checked path below, which raises in the
+        reference's order."""
+        if canvas is not None and self._handle and getattr(self, "_backend", "auto") in ("auto", "triton"):
+            import torch
+
+            packed = _pack_images((*inputs, canvas), self._batch)
+            if packed is not None and packed[3] == torch.cuda.current_device():
+                images, ch, is_float, dev = packed
+                handle = self._handle
+                if (ch, is_float) != (4, False):
+                    handle = self._others.get((ch, is_float)) if self.status.ok() else None
+                if handle:
+                    n = len(images) // 24 - 1
+                    if stream is None:
+                        stream = _current_stream(torch, dev)
+                    elif hasattr(stream, "cuda_stream"):
+                        stream = stream.cuda_stream
+                    s = _raw("hmp_stitcher_process")(handle, images, n, images[24 * n:], stream)
+                    if s.code:
+                        raise CudaStatusError(_status(s))
+                    self._last_handle = handle
+                    return canvas if canvas.dim() == 4 else canvas.unsqueeze(0)
+        return self._run_checked(inputs, canvas, stream)
+
+    def _run_checked(self, inputs: Sequence, canvas=None, stream=None):
         import torch
 
         st = self.status
@@ -769,16 +858,20 @@ class StitchServer:
         return int(cid.value)
 
     def submit(self, config_id: int, inputs: Sequence, canvas) -> int:
-        batched = [_ensure_batched(t) for t in inputs]
-        canvas = _ensure_batched(canvas)
-        imgs = (Image * len(batched))(*[_image(t) for t in batched])
-        cv = _image(canvas)
+        inputs = list(inputs)
         rid = C.c_longlong()
-        st = _status(_lib.lib().hmp_server_submit(self._h, int(config_id), imgs, len(batched), C.byref(cv),
-                                                  C.byref(rid)))
-        if not st.ok():
-            raise CudaStatusError(st)
-        self._live[int(rid.value)] = (batched, canvas)
+        packed = _pack_images((*inputs, canvas), int(canvas.shape[0]) if canvas.dim() == 4 else 1)
+        if packed is not None:
+            images, n = packed[0], len(inputs)
+            s = _raw("hmp_server_submit")(self._h, int(config_id), images, n, images[24 * n:], C.byref(rid))
+        else:
+            batched = [_ensure_batched(t) for t in inputs]
+            cv = _image(_ensure_batched(canvas))
+            imgs = (Image * len(batched))(*[_image(t) for t in batched])
+            s = _lib.lib().hmp_server_submit(self._h, int(config_id), imgs, len(batched), C.byref(cv), C.byref(rid))
+        if s.code:
+            raise CudaStatusError(_status(s))
+        self._live[int(rid.value)] = (inputs, canvas)
         return int(rid.value)
 
     def wait(self, request_id: int, timeout_ms: int = 60000) -> CudaStatus:
