@@ -63,9 +63,9 @@ struct PyrArgs {
   // nullptr: the dense grid.
   const uint32_t* tiles;
   int list_frames;  // listed launches: grid.x = entries x list_frames, frame = blockIdx.x % list_frames
-  // Copy-block mode, pyr_fine: a level-0 pixel whose block of 2^sm_shift pixels is marked in
-  // support_mark ([.][sm_pitch], blend coordinates) lies in a copy block's reconstruction support;
-  // alpha 0 of its label image's pixel there sets *alpha_flag.
+  // Copy-block mode, pyr_fine (two images: pyr_down): a level-0 pixel whose block of 2^sm_shift pixels
+  // is marked in support_mark ([.][sm_pitch], blend coordinates; 1 + slot) lies in a copy block's
+  // reconstruction support; alpha 0 of that slot's pixel there sets *alpha_flag.
   int* alpha_flag;
   const uint8_t* support_mark;
   int sm_pitch, sm_shift;

@@ -214,10 +214,14 @@ __device__ __forceinline__ const uchar4* slot_src_dyn(const PyrArgs& a, int k, i
 // row, its lanes 32 consecutive pixels; the table entries of kBatch pixels are loaded together, then
 // their source pixels. A slot of one image has its frame's base, size and pitch in registers, so a
 // pixel costs a compare and a multiply-add besides its loads. keep: also stored for pyr_fine.
+// kCheck (two images in copy-block mode): a copy block copies slot support_mark - 1 in its support
+// (one byte per 2^(L-1) block), exactly only while every source pixel there has alpha; the canvas
+// gather checks the pixels it reads, and this pass those of the listed tiles, which hold every
+// pyramid-block pixel. (Three and more images: pyr_fine, which reads only the label's pixel.)
 // Before (entries and pixels through cp.async, the frame looked up per pixel) the kernels spent their
 // issue slots on addresses: eight images 9000x2400, 1663 tiles, 64.4 -> 52.5 us; three 6000x1800 FP16,
 // 855 tiles, 32.8 -> 31.2; two 8500x3300, 318 tiles, 18.6 -> 17.2 (alone, cold).
-template <int TD>
+template <int TD, bool kCheck>
 __device__ __forceinline__ void gather_slot(const PyrArgs& a, int k, uint32_t* pk, int X0, int Y0, int b, bool opaque,
                                             bool keep) {
   constexpr int NJ = TD / 32, ROWS = TD / 8, kBatch = 8, kSteps = ROWS * NJ;
@@ -268,6 +272,20 @@ __device__ __forceinline__ void gather_slot(const PyrArgs& a, int k, uint32_t* p
       const int i = (g + u) / NJ, j = (g + u) % NJ;
       pk[(warp + 8 * i) * TD + lane + 32 * j] = v[u];
     }
+    if (kCheck && a.alpha_flag != nullptr) {
+      bool zero = false;
+#pragma unroll
+      for (int u = 0; u < N; ++u) zero = zero || (((in >> u) & 1u) && v[u] < 0x01000000u);
+      if (zero) {
+#pragma unroll 1
+        for (int u = 0; u < N; ++u) {
+          const int x = X0 + lane + 32 * ((g + u) % NJ), y = Y0 + warp + 8 * ((g + u) / NJ);
+          if (((in >> u) & 1u) && pk[(y - Y0) * TD + x - X0] < 0x01000000u &&
+              __ldg(a.support_mark + (long long)(y >> a.sm_shift) * a.sm_pitch + (x >> a.sm_shift)) == k + 1)
+            atomicOr(a.alpha_flag, 1);
+        }
+      }
+    }
     if (keep) {
       uint32_t* d = a.P0[k] + (long long)b * P.w * P.h + (long long)(Y0 + warp - P.y0) * P.w + (X0 + lane - P.x0);
 #pragma unroll
@@ -316,7 +334,7 @@ __global__ void __launch_bounds__(256) pyr_down_kernel(const __grid_constant__ P
     const bool keep = kKeepLevel0 && a.use_p0 && keeps_level0<(NMAX >= 3 || kListed), kWalk>(a);
   #pragma unroll
     for (int k = 0; k < NMAX; ++k)
-      if (active[k]) gather_slot<TD>(a, k, pix + k * TD * TD, X0, Y0, b, opaque, keep);
+      if (active[k]) gather_slot<TD, NMAX == 2 && kListed && !kWalk>(a, k, pix + k * TD * TD, X0, Y0, b, opaque, keep);
     __syncthreads();
     // Levels 1 and 2: one item = one level-2 pixel of one slot = its four level-1 pixels, each the
     // alpha-aware mean of a 2x2 level-0 block (two 8-byte shared loads), summed in (0,0), (1,0),
@@ -425,7 +443,7 @@ __global__ void __launch_bounds__(256) pyr_down_n_kernel(const __grid_constant__
     const bool keep = a.use_p0 && keeps_level0<true, kWalk>(a);
   #pragma unroll 1
     for (int c = 0; c < na; ++c)
-      gather_slot<TD>(a, (list >> (4 * c)) & 15u, pix + c * TD * TD, X0, Y0, b, opaque, keep);
+      gather_slot<TD, false>(a, (list >> (4 * c)) & 15u, pix + c * TD * TD, X0, Y0, b, opaque, keep);
     __syncthreads();
     const bool has2 = L > 2;
     const int lw2 = a.lw[has2 ? 2 : 1], lh2 = a.lh[has2 ? 2 : 1];
@@ -1109,13 +1127,6 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
           // valid label picked otherwise had alpha 0.
           if (a.alpha_flag != nullptr && mv[u] < n && pk != mv[u])
             bad = bad || support_alpha_zero(a, X + (q & 1), Y + (q >> 1), 0u);
-        } else if constexpr (RULE == kRuleTwo && kListed) {
-          // Two images: the support's mark names the slot its copy block copies (1 + slot).
-          if (a.alpha_flag != nullptr && (al[0] == 0.f || al[1] == 0.f)) {
-            const int x = X + (q & 1), y = Y + (q >> 1);
-            const int m = __ldg(a.support_mark + (long long)(y >> a.sm_shift) * a.sm_pitch + (x >> a.sm_shift));
-            bad = bad || (m == 1 && al[0] == 0.f) || (m == 2 && al[1] == 0.f);
-          }
         }
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (pk >= 0) {
@@ -1157,7 +1168,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
                                                  (long long)(py + a.cy_off) * a.C.pitch);
         crow[px + a.cx_off] = pack_rgba(r);
       }
-      if constexpr ((P0M && RULE != kRuleTwo) || (RULE == kRuleTwo && kListed)) {
+      if constexpr (P0M && RULE != kRuleTwo) {
         if (a.alpha_flag != nullptr && __any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(a.alpha_flag, 1);
       }
     }

@@ -161,7 +161,7 @@ struct hmp_stitcher {
   int copy_blocks = 0, empty_blocks = 0, pyramid_blocks = 0;
   long long pyramid_pixels = 0;
   cudaStream_t aux = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_gather = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_gather = nullptr;  // ev_gather: the fallback's order
   double m0_bytes = 0;
   int launches = 0;
   hmp::SrcSet last_src{};  // frames of the last process(), for the pyramid dump
@@ -1114,6 +1114,16 @@ struct hmp_stitcher {
       return cuda_status(err, what);
     };
     hmp::PyrArgs a = pyr_args(S, C);
+    // Copy-block fallback (below): whether this call checks and may need it, whether as one gate
+    // (outside a capture), and whether that gate runs beside the pyramid chain.
+    const bool checked = copy && !copy_opaque;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (checked) {
+      e = cudaStreamIsCapturing(s, &capture);
+      if (e != cudaSuccess) return failed(e, "stream capture query");
+    }
+    const bool gate = checked && capture == cudaStreamCaptureStatusNone;
+    const bool beside = gate && fork && p.n == 2 && n_down[di] > 0;
     if (b5) {
       // Binomial5: the level-by-level chain (its time is reported under pyr_down).
       for (int l = 1; l < p.levels; ++l) a.Rl[l] = Rl[l];
@@ -1167,6 +1177,7 @@ struct hmp_stitcher {
         if (timed) tbegin(1, cs);
         e = hmp::launch_pyr_down(q, p.storage, g, cs);
         if (timed) tend(1, cs);
+        if (e == cudaSuccess && timed && beside) e = cudaEventRecord(ev_gather, cs);  // its alpha checks are in
         if (e != cudaSuccess) return failed(e, "pyr_down launch");
       }
       if (p.levels > 1 && !b5 && (!listed || n_coarse > 0)) {
@@ -1188,7 +1199,7 @@ struct hmp_stitcher {
       }
       return ok_status();
     };
-    if (copy) {  // pyr_fine checks the pyramid-block pixels inside copy blocks' supports
+    if (copy) {  // pyr_fine (two images: pyr_down) checks the pyramid-block pixels inside copy blocks' supports
       a.alpha_flag = copy_opaque ? nullptr : alpha_flag;
       a.support_mark = support_mark;
       a.sm_pitch = sm_pitch;
@@ -1199,20 +1210,20 @@ struct hmp_stitcher {
     // Copy-block fallback, after the gather wrote the copy blocks: it recomputes the whole write
     // rect densely if a copy block's source pixels held alpha 0, and clears the flag. Outside a
     // stream capture it is one thread (hmp_fallback.cu) that returns at once unless the flag is
-    // set, then tail-launches the dense chain; with the gather forked it runs on the pyramid
-    // stream after pyr_fine and the gather, so the caller stream's join follows it directly.
-    // In a CUDA graph the gate's device-side launches did not run (the graph replay test of copy
-    // blocks on alpha-0 frames caught it), so a captured call keeps three gated launches whose
-    // CTAs walk the dense tiles when the flag is set; the last one clears it.
-    // With frames promised opaque (hmp_stitcher_set_copy_blocks mode 2) nothing is checked and no
-    // fallback is launched.
-    const bool checked = copy && !copy_opaque;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (checked) {
-      e = cudaStreamIsCapturing(s, &capture);
-      if (e != cudaSuccess) return failed(e, "stream capture query");
-    }
-    const bool gate = checked && capture == cudaStreamCaptureStatusNone;
+    // set, then tail-launches the dense chain. In a CUDA graph the gate's device-side launches did
+    // not run (the graph replay test of copy blocks on alpha-0 frames caught it), so a captured call
+    // keeps three gated launches whose CTAs walk the dense tiles when the flag is set; the last one
+    // clears it. With frames promised opaque (hmp_stitcher_set_copy_blocks mode 2) nothing is checked
+    // and no fallback is launched.
+    // Where it runs, with the gather forked: two images make both checks before the chain ends (the
+    // gather, and pyr_down instead of pyr_fine), so the gate follows the gather on the caller stream
+    // beside the rest of the chain and its latency is off the critical path (2203x797 L3, two frames:
+    // 37.4 -> 33.0 us a call; 8500x3300 L6: 83.0 -> 82.2). If it launches the dense chain, that
+    // overlaps the listed kernels; every value both write is the same, computed from the same pixels
+    // by the same arithmetic, so neither can read or leave anything else. With more images, whose
+    // pyr_fine checks only the label's pixel and costs less than a check in pyr_down (three images
+    // 91.3 against 93.4 us, eight 196.3 against 199.1), it runs on the pyramid stream after pyr_fine
+    // and the gather, so the caller stream's join follows it directly.
     hmp::PyrArgs f = a;
     f.gate = alpha_flag;
     if (gather) {
@@ -1221,7 +1232,13 @@ struct hmp_stitcher {
       tend(0, s);
       if (e != cudaSuccess) return failed(e, "canvas_gather launch");
     }
-    if (gate && fork) {
+    if (beside) {
+      e = cudaStreamWaitEvent(s, ev_gather, 0);  // recorded after pyr_down
+      f.alpha_flag = nullptr;
+      if (e == cudaSuccess)
+        e = hmp::launch_fallback_gate(f, p.rule, p.storage, tile_down, tile_coarse, dgrid, cgrid, fgrid, coarse_smem, s);
+      if (e != cudaSuccess) return failed(e, "copy-block fallback launch");
+    } else if (gate && fork) {
       e = cudaEventRecord(ev_gather, s);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(aux, ev_gather, 0);
       if (e == cudaSuccess)
