@@ -44,6 +44,18 @@ HMP_HD bool ordered_element(float r, OrderedRun& e) {
   return true;
 }
 
+// The increment of an element that is neither a tie nor too large, without branches; false: it is one of
+// those, and d means nothing.
+HMP_HD bool ordered_plain(float r, int& d) {
+  constexpr float kMagic = 12582912.0f;
+  const float t = r + kMagic;
+  const float f = r - (t - kMagic);
+  int bits;
+  memcpy(&bits, &t, 4);
+  d = int(unsigned(bits) - 0x4B400000u);
+  return (fabsf(r) < 4194304.0f) & (fabsf(f) != 0.5f);
+}
+
 // The units a run adds to a sum of S units (unsigned arithmetic: only partial sums inside the binade
 // are used, the ones past the first failure may wrap).
 HMP_HD int ordered_apply(OrderedRun e, int S) { return int(unsigned(S) + unsigned((S & 1) ? e.d1 : e.d0)); }

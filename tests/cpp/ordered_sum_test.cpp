@@ -29,7 +29,13 @@ static float scanned(const std::vector<float>& x, std::mt19937& rng, long& steps
       size_t i = pos;
       for (; i < end; ++i) {
         hmp::OrderedRun e;
-        if (!hmp::ordered_element(x[i] * scale, e)) break;
+        const bool whole = hmp::ordered_element(x[i] * scale, e);
+        int d = 0;
+        if (hmp::ordered_plain(x[i] * scale, d) != (whole && e.d0 == e.d1) || (whole && e.d0 == e.d1 && d != e.d0)) {
+          std::printf("plain element differs\n");
+          std::exit(1);
+        }
+        if (!whole) break;
         const int n = hmp::ordered_apply(e, P);
         if (!hmp::ordered_inside(n)) break;
         P = n;
