@@ -18,15 +18,15 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
   if (bw <= 0 || bh <= 0 || int(p.mask0.size()) != bw * bh || int(p.slots.size()) != n) return;
   // Level-(L-1) pixel q covers level-0 block q of edge G; per block: the label if uniform, and per
   // image whether every pixel / any pixel has a non-sentinel entry, with the largest coordinates.
-  const int G = 1 << (L - 1);
+  const int sh = L - 1, G = 1 << sh;  // block coordinates by shifts: these loops run over every pixel
   const int gx = (bw + G - 1) / G, gy = (bh + G - 1) / G;
   constexpr uint8_t kUnset = 0xFE, kMixed = 0xFF;
   std::vector<uint8_t> lab(size_t(gx) * gy, kUnset);
   for (int y = 0; y < bh; ++y) {
     const uint8_t* row = &p.mask0[size_t(y) * bw];
-    uint8_t* lb = &lab[size_t(y / G) * gx];
+    uint8_t* lb = &lab[size_t(y >> sh) * gx];
     for (int x = 0; x < bw; ++x) {
-      uint8_t& b = lb[x / G];
+      uint8_t& b = lb[x >> sh];
       if (b == kUnset)
         b = row[x];
       else if (b != row[x])
@@ -58,7 +58,7 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
         const size_t i = size_t(ry) * s.rect.w + rx;
         const uint32_t e = s.map[i];
         const int o = s.owner.empty() ? s.default_owner : s.owner[i];
-        const size_t b = size_t(y / G) * gx + x / G;
+        const size_t b = size_t(y >> sh) * gx + (x >> sh);
         if (two && o == 1) img2_any[b] = 1;
         // Three or more images: each slot holds its own image only.
         if (o >= n || (!two && o != k) || (e & 0xFFFFu) == 0xFFFFu) {

@@ -1281,10 +1281,11 @@ HMP_API hmp_status hmp_stitcher_create(const hmp_config* cfg, hmp_stitcher** out
     rc = HMP_ERR_MEMORY_ALLOCATION;
     msg = "out of host memory while planning";
   }
-  if (rc != HMP_OK)
-    st->status = make_status(rc, msg);
-  else
-    st->status = st->setup();
+  try {
+    st->status = rc != HMP_OK ? make_status(rc, msg) : st->setup();
+  } catch (const std::bad_alloc&) {
+    st->status = make_status(HMP_ERR_MEMORY_ALLOCATION, "out of host memory while planning");
+  }
   if (st->status.code != HMP_OK) {
     // Release device memory now; keep the object for its sticky status.
     for (void* p : st->allocations) cudaFree(p);
