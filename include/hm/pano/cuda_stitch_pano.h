@@ -275,7 +275,7 @@ struct ControlMasksN {
 namespace cuda {
 
 // Pixel types of the reference's pipelines (CudaStitchPano*<T_pipeline, T_compute>): uchar4 is
-// the fused per-frame path; uchar3, float4 and float3 run the level-by-level kernels.
+// the fused per-frame path, uchar3 its own; float4 and float3 run the level-by-level kernels.
 template <typename T>
 struct PixelTraits;
 template <>

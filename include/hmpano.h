@@ -115,9 +115,9 @@ typedef struct hmp_config {
 
 /* Pixel sample types (the reference's CudaStitchPano<T_pipeline, T_compute> pipelines): uchar4 /
  * uchar3 (HMP_PIXEL_U8, canvas packed by truncation) and float4 / float3 (HMP_PIXEL_F32, canvas
- * stores the reconstruction as is). uchar4 runs the fused per-frame kernels; the other three run
- * level-by-level kernels with the same arithmetic (3-channel pixels have no alpha: plain means,
- * plain bilinear upsampling, blends without alpha tests). */
+ * stores the reconstruction as is). uchar4 and uchar3 run fused per-frame kernels of their own, the
+ * float types level-by-level kernels with the same arithmetic (3-channel pixels have no alpha: plain
+ * means, plain bilinear upsampling, blends without alpha tests). */
 #define HMP_PIXEL_U8 0
 #define HMP_PIXEL_F32 1
 
@@ -276,7 +276,9 @@ HMP_API hmp_status hmp_stitcher_set_down_residency(hmp_stitcher* st, int ctas_pe
  * from one single-thread kernel that otherwise returns at once, or under stream capture from three
  * gated launches). Results are identical either way; off forces the full pyramid every call.
  * Applies to RGBA8 stitchers with the box filter and two or more levels: 3..8 images, and two
- * images whose minimised blend strip lines up with the canvas. Mode 2 drops the device check and
+ * images whose minimised blend strip lines up with the canvas. RGB8 stitchers of two or more levels
+ * have copy blocks in any blend region; without alpha they need neither condition, and modes 1 and 2
+ * are the same. Mode 2 drops the device check and
  * its fallback (one launch fewer per call): for frames whose source pixels all have alpha != 0
  * (camera and video frames, alpha 255); a source pixel with alpha 0 behind a copy block then gives
  * that block the source pixel where the reference's pyramid would blend it out. */
