@@ -388,14 +388,4 @@ __device__ __forceinline__ float4 blend_level0(int n, const float4* lap, int v) 
   }
 }
 
-// Read-only loads of a level buffer in HBM (through the non-coherent cache).
-__device__ __forceinline__ float4 ldg_level(const float4* p) { return __ldg(p); }
-__device__ __forceinline__ float4 ldg_level(const half4* p) {
-  const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
-  const __half2 a = *reinterpret_cast<const __half2*>(&raw.x);
-  const __half2 b = *reinterpret_cast<const __half2*>(&raw.y);
-  const float2 fa = __half22float2(a), fb = __half22float2(b);
-  return make_float4(fa.x, fa.y, fb.x, fb.y);
-}
-
 }  // namespace hmp
