@@ -194,6 +194,79 @@ __global__ void __launch_bounds__(256, 6) canvas_gather_kernel(const __grid_cons
   }
 }
 
+// The canvas gather from packed entries, for the calls that may not rewrite the resolved plane
+// (hmp_stitcher.cu): the pixel, fill, skip and alpha rules of resolve_plane_kernel and
+// canvas_gather_kernel, the owners and the frames' bounds looked up per pixel. A warp a 256-pixel row
+// segment, lane l its pixels l + 32j, their loads in flight together; a segment of one owner has its
+// frame in registers. Bound by the issue of the lookups: 8500x3300 hard seam 109 us, against 55 from the
+// resolved plane and 224 where a captured call resolved the plane at every replay.
+__global__ void __launch_bounds__(256, 4) canvas_gather_packed_kernel(const __grid_constant__ GatherArgs a, int opaque,
+                                                                      const __grid_constant__ SkipMap skip) {
+  constexpr int PJ = kSegPixels / 32;
+  const int lane = threadIdx.x & 31;
+  const int x0 = blockIdx.x * kSegPixels + lane, y = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (y >= a.C.h) return;
+  const PlaneDev& P = a.P;
+  const uint32_t* mrow = P.map + (long long)y * P.map_pitch;
+  const uint8_t* orow = P.owner ? P.owner + (long long)y * P.owner_pitch : nullptr;
+  const bool row_skip = y >= a.skip_y0 && y < a.skip_y1;
+  const bool row_chk = a.alpha_flag != nullptr && y >= a.chk_y0 && y < a.chk_y1;
+  const uint8_t* srow = skip.map && y >= skip.wr_y0 && y < skip.wr_y1
+                            ? skip.map + (long long)((y - skip.y0) >> 4) * skip.pitch : nullptr;
+  uint32_t e[PJ];
+  int o[PJ];
+  bool live[PJ];  // stored: inside the canvas and not the pyramid's
+  unsigned lo = 0xFFu, hi = 0u;
+#pragma unroll
+  for (int j = 0; j < PJ; ++j) {
+    const int x = x0 + 32 * j;
+    live[j] = x < a.C.w && !(row_skip && x >= a.skip_x0 && x < a.skip_x1);
+    if (live[j] && srow && x >= skip.wr_x0 && x < skip.wr_x1) live[j] = __ldg(srow + ((x - skip.x0) >> 6)) == 0;
+    e[j] = live[j] ? __ldg(mrow + x) : 0xFFFFFFFFu;
+    o[j] = !live[j] ? 0xFF : (orow ? int(__ldg(orow + x)) : P.default_owner);
+  }
+#pragma unroll
+  for (int j = 0; j < PJ; ++j)
+    if (live[j]) lo = min(lo, unsigned(o[j])), hi = max(hi, unsigned(o[j]));
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  const int one = lo == hi ? int(lo) : 0xFF;
+  bool bad = false;
+  for (int b = 0; b < a.batch; ++b) {
+    uint32_t* crow =
+        reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(a.C.ptr) + b * a.C.bstride + (long long)y * a.C.pitch);
+    uint32_t v[PJ];
+    unsigned read = 0;  // pixels read from a frame, not filled
+    const auto fetch = [&](int j, const char* base, int w, int h, int pitch) {
+      const int sx = int(e[j] & 0xFFFFu), sy = int(e[j] >> 16);
+      v[j] = o[j] < a.n_owners && opaque && sx != 0xFFFF ? 0xFF000000u : 0u;
+      if (o[j] < a.n_owners && sx < w && sy < h) {
+        v[j] = __ldg(reinterpret_cast<const uint32_t*>(base + (long long)sy * pitch) + sx);
+        read |= 1u << j;
+      }
+    };
+    if (one < a.n_owners) {
+      const char* base = reinterpret_cast<const char*>(a.S.ptr[one]) + b * a.S.bstride[one];
+      const int w = a.S.w[one], h = a.S.h[one], pitch = int(a.S.pitch[one]);
+#pragma unroll
+      for (int j = 0; j < PJ; ++j) fetch(j, base, w, h, pitch);
+    } else {
+#pragma unroll
+      for (int j = 0; j < PJ; ++j) {
+        const int k = o[j] < a.n_owners ? o[j] : 0;
+        fetch(j, reinterpret_cast<const char*>(a.S.ptr[k]) + b * a.S.bstride[k], a.S.w[k], a.S.h[k], int(a.S.pitch[k]));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < PJ; ++j) {
+      const int x = x0 + 32 * j;
+      if (live[j]) __stcs(crow + x, v[j]);
+      bad = bad || (row_chk && ((read >> j) & 1u) && v[j] < 0x01000000u && x >= a.chk_x0 && x < a.chk_x1);
+    }
+  }
+  if (a.alpha_flag != nullptr && __any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(a.alpha_flag, 1);
+}
+
 // Resolves one plane's packed entries (raw.map) for the frames' geometry (res, same layout):
 // owner o < n and (sx, sy) inside image o give o << 29 | (sy * pitch / 4 + sx); anything else
 // kOffZero, or kOffOpaque under the soft-seam rule when the owner is valid and sx is not the
@@ -270,6 +343,12 @@ cudaError_t launch_canvas_gather(const GatherArgs& a, bool copy_blocks, cudaStre
     canvas_gather_kernel<true><<<grid, 256, 0, stream>>>(a);
   else
     canvas_gather_kernel<false><<<grid, 256, 0, stream>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_canvas_gather_packed(const GatherArgs& a, bool opaque, const SkipMap& skip, cudaStream_t stream) {
+  const dim3 grid((a.C.w + kSegPixels - 1) / kSegPixels, (a.C.h + 7) / 8);
+  canvas_gather_packed_kernel<<<grid, 256, 0, stream>>>(a, opaque ? 1 : 0, skip);
   return cudaGetLastError();
 }
 

@@ -153,6 +153,9 @@ cudaError_t launch_resolve_plane(const PlaneDev& raw, uint32_t* res, uint8_t* se
 
 // copy_blocks: the plane holds copy-block skips (kOffSkip) or the call checks source alpha.
 cudaError_t launch_canvas_gather(const GatherArgs& a, bool copy_blocks, cudaStream_t stream);
+// The same from the canvas plane's packed entries (a.P: owners and entries as planned, for frames of any
+// geometry; seg_owner unused). opaque: the fill rule of the resolve pass; skip: the call's pyramid blocks.
+cudaError_t launch_canvas_gather_packed(const GatherArgs& a, bool opaque, const SkipMap& skip, cudaStream_t stream);
 
 // Gaussian levels 1..L-1 of every slot; grid = tiles over the blend region x batch.
 cudaError_t launch_pyr_down(const PyrArgs& a, int storage, dim3 grid, cudaStream_t stream);

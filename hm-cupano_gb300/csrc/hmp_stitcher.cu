@@ -121,6 +121,7 @@ struct hmp_stitcher {
   // geometry) and with the planned packed entries it is resolved from.
   hmp::PlaneDev canvas_plane{}, canvas_raw{};
   bool resolved = false;  // canvas_plane holds offsets for the geometry below
+  bool captured = false;  // a captured call reads canvas_plane: it keeps that geometry from then on
   uint8_t* seg_owner = nullptr;  // per 256-pixel canvas row segment, written with the resolve
   int seg_pitch = 0;
   int geo_w[hmp::kDevMaxImages]{}, geo_h[hmp::kDevMaxImages]{};
@@ -1018,17 +1019,29 @@ struct hmp_stitcher {
     last_src = S;
     have_last = true;
     if (generic) return process_generic(S, canvas, s);
-    // RGB8 frames past the resolved offsets' range (byte offsets below 2^29 - 2) take the packed entries.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t ce = cudaStreamIsCapturing(s, &capture);
+    if (ce != cudaSuccess) return cuda_status(ce, "stream capture query");
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    // packed: the gather reads the planned entries. RGB8 frames past the resolved offsets' range (byte
+    // offsets below 2^29 - 2) do, and calls that must not rewrite the plane (below).
     bool packed = false;
     for (int i = 0; rgb && i < p.n; ++i)
       packed = packed || size_t(S.h[i]) * size_t(S.pitch[i]) >= size_t(hmp::kOffMask) - 1;
     if (p.canvas_plane_used && !packed) {
       // The gather reads the canvas plane as offsets into these frames: resolve it for their
-      // geometry on the first call and whenever a size or pitch changes.
+      // geometry on the first call and whenever a size or pitch changes. Only an eager call may: a
+      // captured resolve runs at each replay, not now, so the host would take a plane for resolved
+      // that is not yet, or no longer; and once a captured call reads the plane, every replay needs it
+      // as it was then, so eager calls of another geometry leave it alone.
       bool same = resolved;
       for (int i = 0; i < p.n; ++i)
         same = same && S.w[i] == geo_w[i] && S.h[i] == geo_h[i] && S.pitch[i] == geo_pitch[i];
-      if (!same) {
+      if (same) {
+        captured = captured || capturing;
+      } else if (capturing || captured) {
+        packed = true;
+      } else {
         const cudaError_t re = hmp::launch_resolve_plane(canvas_raw, const_cast<uint32_t*>(canvas_plane.map), seg_owner,
                                                          seg_pitch, S, p.n, p.canvas_opaque && !rgb, rgb,
                                                          copy_plan ? skip : hmp::SkipMap{}, s);
@@ -1060,7 +1073,7 @@ struct hmp_stitcher {
     hmp::GatherArgs ga{};
     if (p.canvas_plane_used) {
       ga.S = S;
-      ga.P = canvas_plane;
+      ga.P = packed ? canvas_raw : canvas_plane;
       ga.C = C;
       ga.batch = p.batch;
       ga.n_owners = p.n;
@@ -1085,10 +1098,14 @@ struct hmp_stitcher {
     // Without copy blocks a write rect covering the canvas leaves the gather nothing to do.
     const bool gather = p.canvas_plane_used &&
                         (p.levels == 0 || copy || p.write.w < p.canvas_w || p.write.h < p.canvas_h);
+    const auto launch_gather = [&] {
+      return packed ? hmp::launch_canvas_gather_packed(ga, p.canvas_opaque, copy ? skip : hmp::SkipMap{}, s)
+                    : hmp::launch_canvas_gather(ga, copy_plan, s);
+    };
     cudaError_t e;
     if (p.levels == 0) {
       tbegin(0, s);
-      e = hmp::launch_canvas_gather(ga, copy_plan, s);
+      e = launch_gather();
       tend(0, s);
       if (timing && tnext < kTimingSlots) ++tnext;
       if (e != cudaSuccess) return cuda_status(e, "canvas_gather launch");
@@ -1117,12 +1134,7 @@ struct hmp_stitcher {
     // Copy-block fallback (below): whether this call checks and may need it, whether as one gate
     // (outside a capture), and whether that gate runs beside the pyramid chain.
     const bool checked = copy && !copy_opaque;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (checked) {
-      e = cudaStreamIsCapturing(s, &capture);
-      if (e != cudaSuccess) return failed(e, "stream capture query");
-    }
-    const bool gate = checked && capture == cudaStreamCaptureStatusNone;
+    const bool gate = checked && !capturing;
     const bool beside = gate && fork && p.n == 2 && n_down[di] > 0;
     if (b5) {
       // Binomial5: the level-by-level chain (its time is reported under pyr_down).
@@ -1228,7 +1240,7 @@ struct hmp_stitcher {
     f.gate = alpha_flag;
     if (gather) {
       tbegin(0, s);
-      e = hmp::launch_canvas_gather(ga, copy_plan, s);
+      e = launch_gather();
       tend(0, s);
       if (e != cudaSuccess) return failed(e, "canvas_gather launch");
     }

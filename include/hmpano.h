@@ -41,7 +41,10 @@
  * the three/N-image seam holds labels 0..n-1). Positions are normalised (minimum 0).
  *
  * All device memory a stitcher needs is allocated by hmp_stitcher_create; process() allocates
- * nothing, so it can be captured in a CUDA graph. One process() may be in flight per stitcher.
+ * nothing, so it can be captured in a CUDA graph, from its first call on, and replayed between calls with
+ * frames of any geometry. (The canvas table resolved for one geometry belongs to the captured call that
+ * read it; calls of another geometry, and a call captured before any eager one of its geometry, read the
+ * table unresolved.) One process() may be in flight per stitcher, replays included.
  */
 #ifndef HMPANO_H
 #define HMPANO_H
@@ -378,9 +381,8 @@ HMP_API void hmp_server_reset_stats(hmp_server* server);
  * under one stream index run in order; different indices run concurrently, so a stitcher's calls
  * must all use one index (HMP_ERR_INVALID_VALUE otherwise). The first capture
  * (hmp_batch_capture, or the first hmp_batch_launch) runs the job once eagerly, then captures it;
- * replays use the device buffers given at add time. Stitchers must outlive the batch, and a
- * stitcher called directly between replays must be given frames of the sizes and pitches it was
- * captured with (a call with other frames re-resolves its canvas table, which the graph reads). */
+ * replays use the device buffers given at add time. Stitchers must outlive the batch; one may
+ * be called directly between replays, with frames of any geometry. */
 typedef struct hmp_batch hmp_batch;
 HMP_API hmp_status hmp_batch_create(hmp_batch** out);
 HMP_API void hmp_batch_destroy(hmp_batch* batch);
