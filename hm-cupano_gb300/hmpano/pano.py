@@ -410,6 +410,25 @@ def _pixel_type(t) -> tuple[int, bool]:
     return int(t.shape[-1]), t.dtype == torch.float32
 
 
+def _checked_type(batched, batch: int) -> tuple[int, bool]:
+    """The one pixel type of inputs that hold `batch` frames each (the native images carry neither)."""
+    if any(t.shape[0] != batch for t in batched):
+        raise ValueError("Input batch size does not match stitcher batch size")
+    if any(t.shape[-1] not in (3, 4) for t in batched):
+        raise ValueError("Only 3- and 4-channel inputs are supported")
+    ptype = _pixel_type(batched[0])
+    if any(_pixel_type(t) != ptype for t in batched):
+        raise ValueError("inputs must share one pixel type")
+    return ptype
+
+
+def _check_canvas(canvas, batch: int, ptype: tuple[int, bool]) -> None:
+    if canvas.shape[0] != batch:
+        raise ValueError("Canvas batch size does not match stitcher batch size")
+    if _pixel_type(canvas) != ptype:
+        raise ValueError("canvas pixel type must match the inputs'")
+
+
 def _image(t) -> Image:
     """hmp_image over a [B, H, W, C] CUDA tensor (C = 4 or 3; uint8 or float32) with dense pixels
     and frames (the row pitch may exceed the row). The stride of a dimension of size 1 is not
@@ -646,13 +665,7 @@ class _Stitcher:
             raise CudaStatusError(st)
         _check_backend(getattr(self, "_backend", "auto"))
         batched = [_ensure_batched(t) for t in inputs]
-        if any(t.shape[0] != self._batch for t in batched):
-            raise ValueError("Input batch size does not match stitcher batch size")
-        if any(t.shape[-1] not in (3, 4) for t in batched):
-            raise ValueError("Only 3- and 4-channel inputs are supported")
-        ptype = _pixel_type(batched[0])
-        if any(_pixel_type(t) != ptype for t in batched):
-            raise ValueError("inputs must share one pixel type")
+        ptype = _checked_type(batched, self._batch)
         handle = self._handle_for(*ptype)
         device = batched[0].device
         if canvas is None:
@@ -660,10 +673,7 @@ class _Stitcher:
                                  dtype=torch.float32 if ptype[1] else torch.uint8, device=device)
         else:
             canvas = _ensure_batched(canvas)
-            if canvas.shape[0] != self._batch:
-                raise ValueError("Canvas batch size does not match stitcher batch size")
-            if _pixel_type(canvas) != ptype:
-                raise ValueError("canvas pixel type must match the inputs'")
+            _check_canvas(canvas, self._batch, ptype)
         imgs = (Image * len(batched))(*[_image(t) for t in batched])
         cv = _image(canvas)
         # The library checks that the current device is the stitcher's; the tensors must live there
@@ -833,7 +843,10 @@ class StitchServer:
         if not st.ok():
             raise CudaStatusError(st)
         self._live = {}
-        self._canvas = {}
+        self._batch = {}  # frames per call, by configuration
+        import torch
+
+        self._device = torch.cuda.current_device()  # the one hmp_server_create took
 
     def close(self) -> None:
         if self._h:
@@ -855,19 +868,30 @@ class StitchServer:
         del keep
         if not st.ok():
             raise CudaStatusError(st)
+        self._batch[int(cid.value)] = int(batch_size)
         return int(cid.value)
 
     def submit(self, config_id: int, inputs: Sequence, canvas) -> int:
+        """A request: the configuration's images and canvas, uint8 RGBA with its frames per call, on the
+        server's device (ValueError otherwise)."""
         inputs = list(inputs)
         rid = C.c_longlong()
-        packed = _pack_images((*inputs, canvas), int(canvas.shape[0]) if canvas.dim() == 4 else 1)
-        if packed is not None:
+        batch = self._batch.get(int(config_id))
+        packed = _pack_images((*inputs, canvas), batch, (4, False))
+        if packed is not None and packed[3] == self._device:
             images, n = packed[0], len(inputs)
             s = _raw("hmp_server_submit")(self._h, int(config_id), images, n, images[24 * n:], C.byref(rid))
         else:
             batched = [_ensure_batched(t) for t in inputs]
-            cv = _image(_ensure_batched(canvas))
+            canvas_b = _ensure_batched(canvas)
+            if any(_pixel_type(t) != (4, False) for t in [*batched, canvas_b]):
+                raise ValueError("a server's images and canvases are uint8 RGBA")
+            if batch is not None and batched:  # the library names an unknown configuration
+                _check_canvas(canvas_b, batch, _checked_type(batched, batch))
+            cv = _image(canvas_b)
             imgs = (Image * len(batched))(*[_image(t) for t in batched])
+            if any(t.device.index != self._device for t in [*batched, canvas_b]):
+                raise ValueError(f"images and canvas must be on the server's CUDA device (cuda:{self._device})")
             s = _lib.lib().hmp_server_submit(self._h, int(config_id), imgs, len(batched), C.byref(cv), C.byref(rid))
         if s.code:
             raise CudaStatusError(_status(s))
