@@ -109,11 +109,14 @@ class Batch:
         self._keep = []
 
     def add(self, stitcher, inputs: Sequence, canvas, stream_index: int = 0) -> None:
+        """One process() call of `stitcher`, whose checks of the batch size and pixel type it makes."""
         batched = [_ensure_batched(t) for t in inputs]
         canvas = _ensure_batched(canvas)
+        ptype = _checked_type(batched, stitcher._batch)
+        _check_canvas(canvas, stitcher._batch, ptype)
         imgs = (Image * len(batched))(*[_image(t) for t in batched])
         cv = _image(canvas)
-        handle = stitcher._handle_for(*_pixel_type(batched[0]))
+        handle = stitcher._handle_for(*ptype)
         self._keep += [batched, canvas, imgs, cv, stitcher]
         s = _status(_lib.lib().hmp_batch_add(self._h, handle, imgs, len(batched), C.byref(cv), int(stream_index)))
         if not s.ok():
