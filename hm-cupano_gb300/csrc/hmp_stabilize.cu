@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
 // are summed tap by tap with the taps outside skipped, and displacements beyond the staged margin
 // read the frames; when the features' mean displacement is far, `next` is staged again around it.
 // The gradients are summed without their factor 1/2, which scales every product and partial sum by a
-// power of two: exact, unless a sum nears the ends of the FP32 range, and then the window is summed
+// power of two: exact, unless a sum nears either end of the FP32 range, and then the window is summed
 // from the frames as written. Bound by the additions' issue (about 24 instructions a tap and pass). 231,496 features of a
 // sub-pixel motion (3840x2160), a thread per feature reading the frames every iteration: 1843 us; so:
 // 395 us, and 16 us to list the features by tile.
@@ -498,11 +498,15 @@ __device__ __forceinline__ void window_time_sums(const float* a, const float* b,
   }
 }
 
-// The step of sums of doubled gradients. in_range: halving them was exact (products far from the ends
-// of the FP32 range; tiny squares mean a determinant below the limit either way).
+// The step of sums of doubled gradients. in_range: the sums proper have the same bits. Doubling scales
+// every product and partial sum exactly except past the ends of the FP32 range: sums that may have
+// overflowed doubled are refused, and so are tiny ones, whose products may be subnormal. (Subnormal
+// products inside a larger sum lie 2^-18 of its last place below it: they can only tip a tie.)
 __device__ __forceinline__ FlowStep flow_step_doubled(float sxx, float syy, float sxy, float stx, float sty,
                                                       bool& in_range) {
-  in_range = fmaxf(fmaxf(sxx, syy), fmaxf(fabsf(stx), fabsf(sty))) < 1e37f && stx == stx && sty == sty;
+  const auto tiny = [](float v) { return v != 0.f && fabsf(v) < 1e-30f; };
+  in_range = fmaxf(fmaxf(sxx, syy), fmaxf(fabsf(stx), fabsf(sty))) < 1e37f && stx == stx && sty == sty &&
+             !(tiny(sxx) || tiny(syy) || tiny(sxy) || tiny(stx) || tiny(sty));
   return flow_step(sxx * 0.25f, syy * 0.25f, sxy * 0.25f, stx * 0.5f, sty * 0.5f);
 }
 
