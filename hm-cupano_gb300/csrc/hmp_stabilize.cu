@@ -703,12 +703,14 @@ __global__ void __launch_bounds__(256) tile_fill_kernel(const int2* xy, const Mo
 // additions, found by scans of whole units (hmp_ordered_sum.h): a chunk of kMotionChunk features is
 // staged in shared memory and scanned at once, up to the first partial sum that leaves the binade;
 // from there `run` elements are added one by one by the thread that found it, and the scan resumes.
-// `run` doubles while scans end close together (sums hovering at a power of two or at zero), as a
-// scan costs about as much as a thousand plain additions, and falls back when one gets far.
-// 11 elements a thread: an odd stride keeps the blocked shared-memory reads free of bank conflicts.
-// Bound by the scans (about 4 us each, issue and barriers). 231,496 features (3840x2160): 746 -> 116 us.
+// A scan costs about as much as 1500 plain additions (3.4 us against 2.2 ns each), so `run` starts at a
+// third of that, doubles while scans end within kMotionFar elements of where they began (sums hovering at
+// a power of two or at zero), and falls back when one gets far; up to kMotionSmall features are summed
+// plainly. 11 elements a thread: an odd stride keeps the blocked shared-memory reads free of bank conflicts.
+// Bound by the scans. One dependent chain against this, 231,000 features at 3840x2160: a moving pair 746
+// and 108 us, a still one, whose sums hover, 839 and about 800; 20,000 unsteady flows 67 and about 70.
 constexpr int kMotionThreads = 1024, kMotionPer = 11, kMotionChunk = kMotionThreads * kMotionPer;
-constexpr int kMotionRunMin = 16, kMotionRunMax = 4096, kMotionFar = 1024;
+constexpr int kMotionRunMin = 512, kMotionRunMax = 8192, kMotionFar = 256, kMotionSmall = 4096;
 
 // Inclusive scan of a warp's runs. Runs without ties (both increments alike in every lane, the usual
 // case) are plain sums: a shuffle and an addition a step instead of two shuffles and a composition
@@ -750,7 +752,7 @@ __global__ void __launch_bounds__(kMotionThreads) motion_kernel(const float2* __
     }
   };
   float s = 0.f;  // the same in every thread
-  int run = kMotionRunMin, last = 0;  // last: the element the previous scan ended at
+  int run = n <= kMotionSmall ? kMotionSmall : kMotionRunMin, last = 0;  // last: the element the present scan began at
   fetch(0);
   for (int base = 0; base < n; base += kMotionChunk) {
     const int cnt = min(kMotionChunk, n - base);
@@ -868,7 +870,7 @@ __global__ void __launch_bounds__(kMotionThreads) motion_kernel(const float2* __
       __syncthreads();
       s = sum_after;
       run = base + at - last < kMotionFar ? min(2 * run, kMotionRunMax) : kMotionRunMin;
-      last = base + at;
+      last = base + end;
       pos = end;
     }
   }
