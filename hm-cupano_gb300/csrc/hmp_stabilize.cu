@@ -384,15 +384,18 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
 // same for every displacement of a window inside both frames, so each later pass over such a window
 // sums only the two that hold the time difference, for the four roundings around the displacement
 // at once (the gradients of a tap are formed once for the four). Windows across the frame's border
-// are summed tap by tap with the taps outside skipped, and displacements beyond the staged margin
-// read the frames; when the features' mean displacement is far, `next` is staged again around it.
+// are summed tap by tap with the taps outside skipped. When the features' mean displacement is past half
+// the margin, `next` is staged again around it; windows beyond the margin take `prev` from its tile and
+// `next` from the frame, by rows (window_far).
 // The gradients are summed without their factor 1/2, which scales every product and partial sum by a
 // power of two: exact, unless a sum nears either end of the FP32 range, and then the window is summed
-// from the frames as written. Bound by the additions' issue (about 24 instructions a tap and pass). 231,496 features of a
-// sub-pixel motion (3840x2160), a thread per feature reading the frames every iteration: 1843 us; so:
-// 395 us, and 16 us to list the features by tile.
+// from the frames as written. Bound by the additions' issue (about 24 instructions a tap and pass).
+// 231,000 features at 3840x2160, window 15, a thread per feature reading the frames every iteration:
+// 1840 us whatever the motion; so: 175 to 385 us for motions up to 4 px, 900 at 6 px, 1290 at 12 px, 1200 at
+// 30 px (1900 with the windows beyond the margin tap by tap from both frames), and 16 us to list the
+// features by tile.
 constexpr int kFlowTile = 64, kFlowPitch = 96, kFlowThreads = 128;
-constexpr int kFlowMaxHalf = 10;
+constexpr int kFlowMaxHalf = 10, kFlowFewFar = 6;
 __host__ __device__ constexpr int flow_margin(int half) { return (kFlowPitch - kFlowTile) / 2 - half; }  // so `next` is 96 x 96
 __host__ __device__ constexpr int flow_prev_rows(int half) { return kFlowTile + 2 * half + 2; }
 __host__ __device__ constexpr int flow_smem(int half) { return (flow_prev_rows(half) + kFlowPitch) * kFlowPitch * int(sizeof(float)); }
@@ -498,6 +501,91 @@ __device__ __forceinline__ void window_time_sums(const float* a, const float* b,
   }
 }
 
+// W values of a row of a frame from value L on, by aligned 16-byte loads (a warp's windows lie scattered:
+// a load of four values costs the L1 what one of a single value does); inside: every chunk lies in the
+// frame's `total` values, else value by value, 0 outside.
+template <int W>
+struct FarRow {
+  static constexpr int NC = (W + 6) / 4;  // chunks: up to 3 values before the row's first
+  static_assert(W + 3 <= 4 * NC, "whole rows");
+  float4 c[NC];
+  int off;
+  __device__ __forceinline__ void load(const float* __restrict__ frame, long long total, long long L) {
+    off = int(reinterpret_cast<uintptr_t>(frame + L) >> 2) & 3;
+    const long long at = L - off;
+    if (at >= 0 && at + 4 * NC <= total) {
+#pragma unroll
+      for (int k = 0; k < NC; ++k) c[k] = __ldg(reinterpret_cast<const float4*>(frame + at) + k);
+    } else {
+      const auto one = [&](long long i) { return i >= 0 && i < total ? __ldg(frame + i) : 0.f; };
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const long long i = at + 4 * k;
+        c[k] = make_float4(one(i), one(i + 1), one(i + 2), one(i + 3));
+      }
+    }
+  }
+  __device__ __forceinline__ void values(float (&v)[W]) const {
+    const auto at = [&](int i) {
+      const float4 q = c[i >> 2];
+      return (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
+    };
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const float lo = off & 1 ? at(i + 1) : at(i), hi = off & 1 ? at(i + 3) : at(i + 2);
+      v[i] = off & 2 ? hi : lo;
+    }
+  }
+};
+
+// The sums of a window whose displacement the staged part of `next` does not cover: `prev` from its tile
+// (a as above), `next` from the frame, its window's first tap at (x0, y0), a row ahead of the sums. Without
+// kMask, of a window inside both frames: the time sums only; with it all five, over the taps of set bits.
+template <int W, bool kMask>
+__device__ __forceinline__ void window_far(const float* a, const float* __restrict__ next, int x0, int y0, int w, int h,
+                                           unsigned cm, unsigned rm, float& sxx, float& syy, float& sxy, float& stx,
+                                           float& sty) {
+  constexpr bool kAhead = W <= 15;  // larger windows have no registers for two rows of `next`
+  const long long total = (long long)w * h;
+  float up[W + 2], mid[W + 2], dn[W + 2], n[W];
+  FarRow<W> ahead;
+  const auto request = [&](int j) {
+    if (!kMask || ((rm >> j) & 1u)) ahead.load(next, total, (long long)(y0 + j) * w + x0);
+  };
+  if (kAhead) request(0);
+#pragma unroll
+  for (int c = 0; c < W + 2; ++c) up[c] = a[c], mid[c] = a[kFlowPitch + c];
+  if (kMask) sxx = syy = sxy = 0.f;
+  stx = sty = 0.f;
+#pragma unroll 1
+  for (int j = 0; j < W; ++j) {
+    const float* d = a + (j + 2) * kFlowPitch;
+#pragma unroll
+    for (int c = 0; c < W + 2; ++c) dn[c] = d[c];
+    const unsigned row = kMask ? (((rm >> j) & 1u) ? cm : 0u) : 0u;
+    if (!kAhead) request(j);
+    ahead.values(n);
+    if (kAhead && j + 1 < W) request(j + 1);
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const float ix = mid[i + 2] - mid[i];
+      const float iy = dn[i + 1] - up[i + 1];
+      const float it = n[i] - mid[i + 1];
+      if (!kMask || ((row >> i) & 1u)) {
+        if (kMask) {
+          sxx += ix * ix;
+          syy += iy * iy;
+          sxy += ix * iy;
+        }
+        stx += ix * it;
+        sty += iy * it;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < W + 2; ++c) up[c] = mid[c], mid[c] = dn[c];
+  }
+}
+
 // The step of sums of doubled gradients. in_range: the sums proper have the same bits. Doubling scales
 // every product and partial sum exactly except past the ends of the FP32 range: sums that may have
 // overflowed doubled are refused, and so are tiny ones, whose products may be subnormal. (Subnormal
@@ -515,6 +603,12 @@ __device__ __forceinline__ unsigned range_mask(int lo, int hi, int W) {
   lo = max(lo, 0);
   hi = min(hi, W);
   return hi > lo ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+}
+
+// The plain window where the tiled kernel seldom needs it, out of its way.
+__device__ __noinline__ FlowStep window_global_call(const float* __restrict__ prev, const float* __restrict__ next, int2 p,
+                                                    int rdx, int rdy, int half, int w, int h) {
+  return window_global(prev, next, p, rdx, rdy, half, w, h);
 }
 
 template <int HALF>
@@ -598,7 +692,7 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
       }
       bool in_range;
       zero = flow_step_doubled(sxx, syy, sxy, stx, sty, in_range);
-      if (!in_range) zero = window_global(prev, next, p, 0, 0, HALF, w, h);
+      if (!in_range) zero = window_global_call(prev, next, p, 0, 0, HALF, w, h);
     }
     bool recentred = false;
     while (true) {
@@ -633,11 +727,15 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
         }
       }
       if (!__any_sync(0xFFFFFFFFu, need)) break;
-      if (!need) continue;
+      // A warp's windows beyond the staged part wait for those inside it, where they are more than a few: then
+      // they are summed together, not beside one of the others pass after pass.
+      const bool near1 = abs(rx - cx) <= M && abs(ry - cy) <= M;
+      const unsigned far_lanes = __ballot_sync(0xFFFFFFFFu, need && !near1);
+      const bool defer = __any_sync(0xFFFFFFFFu, need && near1) && __popc(far_lanes) > kFlowFewFar;
+      if (!need || (defer && !near1)) continue;
       // The rounding and its neighbours toward the match the last step pointed at: iterations near a
       // match add the same step until the rounding crosses to that side.
       const int bx = st.ex < float(rx) ? rx - 1 : rx, by = st.ey < float(ry) ? ry - 1 : ry;
-      const bool near1 = abs(rx - cx) <= M && abs(ry - cy) <= M;
       const bool near4 = near1 && bx - cx >= -M && bx + 1 - cx <= M && by - cy >= -M && by + 1 - cy <= M;
       qb = qa;
       if (inside && near4 && p.x - HALF + bx >= 0 && p.x + HALF + bx + 1 < w - 1 && p.y - HALF + by >= 0 &&
@@ -652,7 +750,7 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
         for (int q = 0; q < 4; ++q) {
           bool in_range;
           FlowStep s = flow_step_doubled(sxx, syy, sxy, stx[q], sty[q], in_range);
-          if (!in_range) s = window_global(prev, next, p, bx + (q & 1), by + (q >> 1), HALF, w, h);
+          if (!in_range) s = window_global_call(prev, next, p, bx + (q & 1), by + (q >> 1), HALF, w, h);
           qa.x[q] = s.x;
           qa.y[q] = s.y;
           if (s.bad) qa.bad |= 1u << q;
@@ -664,10 +762,22 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
         window_sums<W, true>(a, sn + (ly + ry - cy + M) * P + lx + rx - cx + M, cm, rm, a0, a1, a2, stx, sty);
         bool in_range;
         FlowStep s = flow_step_doubled(a0, a1, a2, stx, sty, in_range);
-        if (!in_range) s = window_global(prev, next, p, rx, ry, HALF, w, h);
+        if (!in_range) s = window_global_call(prev, next, p, rx, ry, HALF, w, h);
         qa.set(rx, ry, s);
       } else {
-        qa.set(rx, ry, window_global(prev, next, p, rx, ry, HALF, w, h));
+        const int x0 = p.x - HALF + rx, y0 = p.y - HALF + ry;
+        float a0 = sxx, a1 = syy, a2 = sxy, stx, sty;
+        if (inside && x0 >= 0 && x0 + W < w && y0 >= 0 && y0 + W < h) {
+          window_far<W, false>(a, next, x0, y0, w, h, 0u, 0u, a0, a1, a2, stx, sty);
+        } else {
+          unsigned cm, rm;
+          masks(rx, ry, cm, rm);
+          window_far<W, true>(a, next, x0, y0, w, h, cm, cm != 0u ? rm : 0u, a0, a1, a2, stx, sty);
+        }
+        bool in_range;
+        FlowStep s = flow_step_doubled(a0, a1, a2, stx, sty, in_range);
+        if (!in_range) s = window_global_call(prev, next, p, rx, ry, HALF, w, h);
+        qa.set(rx, ry, s);
       }
     }
     if (f >= 0) flow[f] = make_float2(st.dx, st.dy);
