@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
   flow[f] = make_float2(st.dx, st.dy);
 }
 
-// Windows of 3 to 21 pixels: a CTA per 64 x 64 tile of the frame, its features one to a thread, the
+// Windows of 3 to 21 pixels: a CTA per 64 x 64 tile of the frame (and 128 features), one to a thread, the
 // tile of `prev` (with the window's halo and the gradients') and of `next` (with the window's halo
 // and kFlowMargin pixels of motion) in shared memory. Features of a warp sit at scattered places, so
 // their taps are 4-byte accesses at unrelated addresses: from L1 each costs a wavefront per lane,
@@ -611,40 +611,48 @@ __device__ __noinline__ FlowStep window_global_call(const float* __restrict__ pr
   return window_global(prev, next, p, rdx, rdy, half, w, h);
 }
 
+// What the tiled flow's kernels share besides the features: per tile the count of its features and where
+// they end in `order`; the work items, a tile and which kFlowThreads of its features, so that a crowded tile
+// is shared by many CTAs (20,000 features in one: 2100 us for a call as rounds of one CTA, 127 so).
+struct FlowItems {
+  int* cnt;
+  int* at;
+  int* order;
+  int2* items;
+  int* n_items;  // [0] the number, [1] how many were taken besides the CTAs' first ones
+};
+
 template <int HALF>
 __global__ void __launch_bounds__(kFlowThreads, 3)
     flow_tile_kernel(const float* __restrict__ prev, const float* __restrict__ next, const int2* __restrict__ xy,
-                     const int* __restrict__ order, const int* __restrict__ tile_cnt, const int* __restrict__ tile_end,
-                     int w, int h, float2* flow) {
+                     const __grid_constant__ FlowItems q, int tiles_x, int w, int h, float2* flow) {
   constexpr int W = 2 * HALF + 1, M = flow_margin(HALF), P = kFlowPitch;
   extern __shared__ float tiles[];
   float* sp = tiles;                             // prev, origin (X0 - HALF - 1, Y0 - HALF - 1)
   float* sn = tiles + flow_prev_rows(HALF) * P;  // next, origin (X0 - HALF + cx - M, Y0 - HALF + cy - M)
-  __shared__ int bank_cnt[32], slot[kFlowThreads], mean_sum[3];
-  const int tile = blockIdx.y * gridDim.x + blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  const int total = tile_cnt[tile];
-  if (total == 0) return;
-  const int first = tile_end[tile] - total;
-  const int X0 = blockIdx.x * kFlowTile, Y0 = blockIdx.y * kFlowTile;
-  int cx = 0, cy = 0;  // the displacement `next` is staged around
-  stage_frame(sp, prev, X0 - HALF - 1, Y0 - HALF - 1, flow_prev_rows(HALF), flow_prev_rows(HALF), w, h);
-  stage_frame(sn, next, X0 - HALF - M, Y0 - HALF - M, P, P, w, h);
-  const int rounds = (total + kFlowThreads - 1) / kFlowThreads, per = (total + rounds - 1) / rounds;
-  for (int r0 = 0; r0 < total; r0 += per) {
-    const int nc = min(per, total - r0);
-    if (cx != 0 || cy != 0) {  // every window starts without displacement
-      cx = cy = 0;
-      __syncthreads();
-      stage_frame(sn, next, X0 - HALF - M, Y0 - HALF - M, P, P, w, h);
-    }
-    // Deal the features out by bank.
+  __shared__ int bank_cnt[32], slot[kFlowThreads], mean_sum[3], taken;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (int(blockIdx.x) >= q.n_items[0]) return;
+  for (bool first_item = true;; first_item = false) {  // item blockIdx.x, then the next that no CTA has
+    __syncthreads();  // the last item is done with shared memory
+    if (tid == 0) taken = first_item ? int(blockIdx.x) : int(gridDim.x) + atomicAdd(q.n_items + 1, 1);
     if (tid < 32) bank_cnt[tid] = 0;
     if (tid < 3) mean_sum[tid] = 0;
     slot[tid] = -1;
     __syncthreads();
+    if (taken >= q.n_items[0]) return;
+    const int2 item = q.items[taken];
+    const int total = q.cnt[item.x], rounds = (total + kFlowThreads - 1) / kFlowThreads;
+    const int per = (total + rounds - 1) / rounds, r0 = item.y * per, nc = min(per, total - r0);
+    const int first = q.at[item.x] - total + r0;
+    const int X0 = item.x % tiles_x * kFlowTile, Y0 = item.x / tiles_x * kFlowTile;
+    int cx = 0, cy = 0;  // the displacement `next` is staged around
+    stage_frame(sp, prev, X0 - HALF - 1, Y0 - HALF - 1, flow_prev_rows(HALF), flow_prev_rows(HALF), w, h);
+    stage_frame(sn, next, X0 - HALF - M, Y0 - HALF - M, P, P, w, h);
+    // Deal the features out by bank.
     int mine = -1, bank = 0, rank = 0;
     if (tid < nc) {
-      mine = order[first + r0 + tid];
+      mine = q.order[first + tid];
       bank = xy[mine].x & 31;
       rank = atomicAdd(&bank_cnt[bank], 1);
     }
@@ -665,10 +673,10 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
       slot[(pos % warps) * 32 + pos / warps] = mine;
     }
     stage_wait();  // the tiles and the slots
-    const int f = slot[tid];
-    const int2 p = f >= 0 ? xy[f] : make_int2(X0, Y0);
-    const int lx = p.x - X0, ly = p.y - Y0;
-    const float* a = sp + ly * P + lx;
+    const bool has = slot[tid] >= 0;
+    const int2 p = has ? xy[slot[tid]] : make_int2(X0, Y0);
+    const int own = (p.y - Y0) * P + p.x - X0;  // the feature's place in the tile
+    const float* a = sp + own;
     const bool inside = p.x - HALF >= 1 && p.x + HALF < w - 1 && p.y - HALF >= 1 && p.y + HALF < h - 1;
     // Bits of the window's taps that lie inside both frames under displacement (rx, ry).
     const auto masks = [&](int rx, int ry, unsigned& cm, unsigned& rm) {
@@ -679,10 +687,10 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
     FlowStep zero{0.f, 0.f, true};
     FlowQuad qa, qb;
     float sxx = 0.f, syy = 0.f, sxy = 0.f;
-    if (f < 0) st.iter = 10;
-    if (f >= 0) {
+    if (!has) st.iter = 10;
+    if (has) {
       float stx, sty;
-      const float* b = sn + (ly + M) * P + lx + M;
+      const float* b = sn + own + M * P + M;
       if (__all_sync(__activemask(), inside)) {
         window_sums<W, false>(a, b, 0u, 0u, sxx, syy, sxy, stx, sty);
       } else {
@@ -741,7 +749,7 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
       if (inside && near4 && p.x - HALF + bx >= 0 && p.x + HALF + bx + 1 < w - 1 && p.y - HALF + by >= 0 &&
           p.y + HALF + by + 1 < h - 1) {
         float stx[4], sty[4];
-        window_time_sums<W>(a, sn + (ly + by - cy + M) * P + lx + bx - cx + M, stx, sty);
+        window_time_sums<W>(a, sn + own + (by - cy + M) * P + bx - cx + M, stx, sty);
         qa.x0 = bx;
         qa.y0 = by;
         qa.have = 15u;
@@ -759,7 +767,7 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
         unsigned cm, rm;
         masks(rx, ry, cm, rm);
         float a0, a1, a2, stx, sty;
-        window_sums<W, true>(a, sn + (ly + ry - cy + M) * P + lx + rx - cx + M, cm, rm, a0, a1, a2, stx, sty);
+        window_sums<W, true>(a, sn + own + (ry - cy + M) * P + rx - cx + M, cm, rm, a0, a1, a2, stx, sty);
         bool in_range;
         FlowStep s = flow_step_doubled(a0, a1, a2, stx, sty, in_range);
         if (!in_range) s = window_global_call(prev, next, p, rx, ry, HALF, w, h);
@@ -780,31 +788,34 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
         qa.set(rx, ry, s);
       }
     }
-    if (f >= 0) flow[f] = make_float2(st.dx, st.dy);
-    __syncthreads();  // slot, bank_cnt and the tiles are free for the next round
+    if (has) flow[slot[tid]] = make_float2(st.dx, st.dy);
   }
 }
 
 // Grids of the per-feature passes: the feature count is known on the device only and the capacity
 // may be every pixel, so a few CTAs per SM walk the features.
 constexpr unsigned kFeatureBlocks = 152 * 4;
+constexpr unsigned kFlowBlocks = 152 * 3;  // flow_tile_kernel's, as many as are resident
 
-// Features by tile: their counts, then (after corner_scan_kernel's offsets) their indices, tile by
-// tile. The order inside a tile is left to the atomics; a feature's flow does not depend on it.
-__global__ void __launch_bounds__(256) tile_count_kernel(const int2* xy, const Motion* m, int cap, int tiles_x, int* cnt) {
+// Features by tile: their counts and the work items (each kFlowThreads-th feature of a tile opens one),
+// then (after corner_scan_kernel's offsets) their indices, tile by tile. The order inside a tile is left to
+// the atomics; a feature's flow does not depend on it.
+__global__ void __launch_bounds__(256) tile_count_kernel(const int2* xy, const Motion* m, int cap, int tiles_x,
+                                                         const __grid_constant__ FlowItems q) {
   const int n = min(m->corners, cap);
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
     const int2 p = xy[f];
-    atomicAdd(&cnt[(p.y / kFlowTile) * tiles_x + p.x / kFlowTile], 1);
+    const int tile = (p.y / kFlowTile) * tiles_x + p.x / kFlowTile, i = atomicAdd(q.cnt + tile, 1);
+    if (i % kFlowThreads == 0) q.items[atomicAdd(q.n_items, 1)] = make_int2(tile, i / kFlowThreads);
   }
 }
 
-__global__ void __launch_bounds__(256) tile_fill_kernel(const int2* xy, const Motion* m, int cap, int tiles_x, int* at,
-                                                        int* order) {
+__global__ void __launch_bounds__(256) tile_fill_kernel(const int2* xy, const Motion* m, int cap, int tiles_x,
+                                                        const __grid_constant__ FlowItems q) {
   const int n = min(m->corners, cap);
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
     const int2 p = xy[f];
-    order[atomicAdd(&at[(p.y / kFlowTile) * tiles_x + p.x / kFlowTile], 1)] = f;
+    q.order[atomicAdd(&q.at[(p.y / kFlowTile) * tiles_x + p.x / kFlowTile], 1)] = f;
   }
 }
 
@@ -1050,16 +1061,15 @@ struct hmp_stabilizer {
   Motion* motion = nullptr;
   float* temp = nullptr;  // an in-place warp's output before the copy back
   int tiles_x = 0, tiles = 0;  // flow tiles of the frame
-  int* tile_cnt = nullptr;     // features per flow tile
-  int* tile_at = nullptr;      // where a tile's features start in `order` (their end once filled)
-  int* order = nullptr;        // feature indices, tile by tile
+  FlowItems items{};           // `cnt` and, after it, `n_items` are cleared together
   ~hmp_stabilizer() {
     for (void* p : {static_cast<void*>(resp), static_cast<void*>(corner_bits), static_cast<void*>(row_cnt), static_cast<void*>(row_off),
                     static_cast<void*>(xy), static_cast<void*>(flow), static_cast<void*>(motion),
-                    static_cast<void*>(temp), static_cast<void*>(tile_cnt), static_cast<void*>(tile_at),
-                    static_cast<void*>(order)})
+                    static_cast<void*>(temp), static_cast<void*>(items.cnt), static_cast<void*>(items.at),
+                    static_cast<void*>(items.order), static_cast<void*>(items.items)})
       if (p) cudaFree(p);
   }
+  int most_items() const { return tiles + cap / kFlowThreads; }
   hmp_status check(const void* a, const void* b) const {
     int dev = -1;
     cudaGetDevice(&dev);
@@ -1074,9 +1084,9 @@ namespace {
 // flow_tile_kernel by half window (nullptr: none).
 template <int HALF>
 void launch_flow_tile(const hmp_stabilizer& st, const float* prev, const float* next, cudaStream_t cs) {
-  const dim3 grid(st.tiles_x, st.tiles / st.tiles_x);
-  flow_tile_kernel<HALF><<<grid, kFlowThreads, flow_smem(HALF), cs>>>(prev, next, st.xy, st.order, st.tile_cnt,
-                                                                      st.tile_at, st.w, st.h, st.flow);
+  const unsigned grid = std::min(unsigned(st.most_items()), kFlowBlocks);
+  flow_tile_kernel<HALF><<<grid, kFlowThreads, flow_smem(HALF), cs>>>(prev, next, st.xy, st.items, st.tiles_x, st.w,
+                                                                      st.h, st.flow);
 }
 
 using FlowTileLaunch = void (*)(const hmp_stabilizer&, const float*, const float*, cudaStream_t);
@@ -1123,9 +1133,11 @@ HMP_API hmp_status hmp_stabilizer_create(int width, int height, int max_features
   if (e == cudaSuccess) e = cudaMalloc(&st->flow, size_t(std::max(st->cap, 1)) * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&st->motion, sizeof(Motion));
   if (e == cudaSuccess) e = cudaMalloc(&st->temp, px * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&st->tile_cnt, size_t(st->tiles) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&st->tile_at, size_t(st->tiles) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&st->order, size_t(std::max(st->cap, 1)) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&st->items.cnt, size_t(st->tiles + 2) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&st->items.at, size_t(st->tiles) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&st->items.order, size_t(std::max(st->cap, 1)) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&st->items.items, size_t(st->most_items()) * sizeof(int2));
+  if (e == cudaSuccess) st->items.n_items = st->items.cnt + st->tiles;
   if (e == cudaSuccess) e = flow_tile_init();
   if (e == cudaSuccess) e = cudaMemset(st->motion, 0, sizeof(Motion));
   if (e != cudaSuccess) {
@@ -1165,12 +1177,12 @@ HMP_API hmp_status hmp_stabilizer_flow(hmp_stabilizer* st, const float* prev, co
   const unsigned blocks = unsigned((std::max(st->cap, 1) + 255) / 256);
   const int half = window_size / 2;
   if (half >= 1 && half <= kFlowMaxHalf) {
-    cudaError_t e = cudaMemsetAsync(st->tile_cnt, 0, size_t(st->tiles) * sizeof(int), cs);
+    cudaError_t e = cudaMemsetAsync(st->items.cnt, 0, size_t(st->tiles + 2) * sizeof(int), cs);
     if (e != cudaSuccess) return cuda_failure(e, "flow set-up");
     const unsigned strided = std::min(blocks, kFeatureBlocks);
-    tile_count_kernel<<<strided, 256, 0, cs>>>(st->xy, st->motion, st->cap, st->tiles_x, st->tile_cnt);
-    corner_scan_kernel<<<1, 1024, 0, cs>>>(st->tile_cnt, st->tiles, st->tile_at, nullptr);
-    tile_fill_kernel<<<strided, 256, 0, cs>>>(st->xy, st->motion, st->cap, st->tiles_x, st->tile_at, st->order);
+    tile_count_kernel<<<strided, 256, 0, cs>>>(st->xy, st->motion, st->cap, st->tiles_x, st->items);
+    corner_scan_kernel<<<1, 1024, 0, cs>>>(st->items.cnt, st->tiles, st->items.at, nullptr);
+    tile_fill_kernel<<<strided, 256, 0, cs>>>(st->xy, st->motion, st->cap, st->tiles_x, st->items);
     kFlowTileLaunch[half](*st, prev, next, cs);
   } else {
     flow_kernel<<<blocks, 256, 0, cs>>>(prev, next, st->xy, st->motion, st->cap, st->w, st->h, half, st->flow);
