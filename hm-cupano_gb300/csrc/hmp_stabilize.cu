@@ -345,7 +345,8 @@ __device__ __forceinline__ FlowStep window_global(const float* __restrict__ prev
 }
 
 // Any window: a thread per feature, every tap from the frames. The last four roundings' steps are
-// kept.
+// kept. Windows of 3 too: nine taps cost less than listing the features by tile and staging the tiles
+// (a call on 3840x2160, 231,000 features 430 -> 300 us; 4000 at 12 px on 1920x1080 112 -> 62).
 __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ prev, const float* __restrict__ next,
                                                    const int2* xy, const Motion* m, int cap, int w, int h, int half,
                                                    float2* flow) {
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
   flow[f] = make_float2(st.dx, st.dy);
 }
 
-// Windows of 3 to 21 pixels: a CTA per 64 x 64 tile of the frame (and 128 features), one to a thread, the
+// Windows of 5 to 21 pixels: a CTA per 64 x 64 tile of the frame (and 128 features), one to a thread, the
 // tile of `prev` (with the window's halo and the gradients') and of `next` (with the window's halo
 // and kFlowMargin pixels of motion) in shared memory. Features of a warp sit at scattered places, so
 // their taps are 4-byte accesses at unrelated addresses: from L1 each costs a wavefront per lane,
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
 // 30 px (1900 with the windows beyond the margin tap by tap from both frames), and 16 us to list the
 // features by tile.
 constexpr int kFlowTile = 64, kFlowPitch = 96, kFlowThreads = 128;
-constexpr int kFlowMaxHalf = 10, kFlowFewFar = 6;
+constexpr int kFlowMinHalf = 2, kFlowMaxHalf = 10, kFlowFewFar = 6;
 __host__ __device__ constexpr int flow_margin(int half) { return (kFlowPitch - kFlowTile) / 2 - half; }  // so `next` is 96 x 96
 __host__ __device__ constexpr int flow_prev_rows(int half) { return kFlowTile + 2 * half + 2; }
 __host__ __device__ constexpr int flow_smem(int half) { return (flow_prev_rows(half) + kFlowPitch) * kFlowPitch * int(sizeof(float)); }
@@ -1091,14 +1092,14 @@ void launch_flow_tile(const hmp_stabilizer& st, const float* prev, const float* 
 
 using FlowTileLaunch = void (*)(const hmp_stabilizer&, const float*, const float*, cudaStream_t);
 constexpr FlowTileLaunch kFlowTileLaunch[kFlowMaxHalf + 1] = {
-    nullptr,             launch_flow_tile<1>, launch_flow_tile<2>, launch_flow_tile<3>, launch_flow_tile<4>, launch_flow_tile<5>,
+    nullptr,             nullptr,             launch_flow_tile<2>, launch_flow_tile<3>, launch_flow_tile<4>, launch_flow_tile<5>,
     launch_flow_tile<6>, launch_flow_tile<7>, launch_flow_tile<8>, launch_flow_tile<9>, launch_flow_tile<10>};
 
 template <int HALF = kFlowMaxHalf>
 cudaError_t flow_tile_init() {
   const cudaError_t e =
       cudaFuncSetAttribute(flow_tile_kernel<HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, flow_smem(HALF));
-  if constexpr (HALF > 1) {
+  if constexpr (HALF > kFlowMinHalf) {
     return e == cudaSuccess ? flow_tile_init<HALF - 1>() : e;
   } else {
     return e;
@@ -1176,7 +1177,7 @@ HMP_API hmp_status hmp_stabilizer_flow(hmp_stabilizer* st, const float* prev, co
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   const unsigned blocks = unsigned((std::max(st->cap, 1) + 255) / 256);
   const int half = window_size / 2;
-  if (half >= 1 && half <= kFlowMaxHalf) {
+  if (half >= kFlowMinHalf && half <= kFlowMaxHalf) {
     cudaError_t e = cudaMemsetAsync(st->items.cnt, 0, size_t(st->tiles + 2) * sizeof(int), cs);
     if (e != cudaSuccess) return cuda_failure(e, "flow set-up");
     const unsigned strided = std::min(blocks, kFeatureBlocks);
