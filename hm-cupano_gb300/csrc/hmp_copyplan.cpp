@@ -5,6 +5,76 @@
 
 namespace hmp {
 
+// The coarse and down lists of the pyramid blocks in cp.fine_list.
+static void list_tiles(const Plan& p, int td, int t1, CopyPlan& cp) {
+  const int L = p.levels, bw = p.lw[0], bh = p.lh[0];
+  const int wx0 = p.write.x - p.blend.x, wy0 = p.write.y - p.blend.y;
+  const int wx1 = wx0 + p.write.w, wy1 = wy0 + p.write.h;
+  cp.coarse_list.clear();
+  cp.down_list.clear();
+  // Level-1 tiles whose R^1 the pyramid blocks read (pyr_fine's 33 x 9 level-1 tile from
+  // (bx0 / 2, by0 / 2), coordinates clamped to the level), and level-0 tiles whose G^l levels (or
+  // kept level-0 pixels) pyr_fine and pyr_coarse read.
+  const int lw1 = p.lw[1], lh1 = p.lh[1];
+  const int ncx = (lw1 + t1 - 1) / t1, ncy = (lh1 + t1 - 1) / t1;
+  const int ndx = (bw + td - 1) / td, ndy = (bh + td - 1) / td;
+  cp.dense_coarse = (long long)ncx * ncy;
+  cp.dense_down = (long long)ndx * ndy;
+  std::vector<uint8_t> cmark(size_t(ncx) * ncy, 0), dmark(size_t(ndx) * ndy, 0);
+  const auto mark_down = [&](int lx0, int ly0, int lx1, int ly1) {  // level-0 pixels, inclusive
+    lx0 = std::max(lx0, 0);
+    ly0 = std::max(ly0, 0);
+    lx1 = std::min(lx1, bw - 1);
+    ly1 = std::min(ly1, bh - 1);
+    for (int ty = ly0 / td; ty <= ly1 / td; ++ty)
+      for (int tx = lx0 / td; tx <= lx1 / td; ++tx) dmark[size_t(ty) * ndx + tx] = 1;
+  };
+  for (uint32_t f : cp.fine_list) {
+    const int bx0 = cp.fx0 + 64 * int(f & 0xFFFFu), by0 = cp.fy0 + 16 * int(f >> 16);
+    const int tx0 = bx0 >> 1, ty0 = by0 >> 1;
+    const int tx1 = std::min(tx0 + 32, lw1 - 1), ty1 = std::min(ty0 + 8, lh1 - 1);
+    for (int ty = ty0 / t1; ty <= ty1 / t1; ++ty)
+      for (int tx = tx0 / t1; tx <= tx1 / t1; ++tx) cmark[size_t(ty) * ncx + tx] = 1;
+    mark_down(2 * tx0, 2 * ty0, 2 * tx1 + 1, 2 * ty1 + 1);  // G^1 taps; the block's own pixels lie inside
+  }
+  for (int ty = 0; ty < ncy; ++ty)
+    for (int tx = 0; tx < ncx; ++tx) {
+      if (!cmark[size_t(ty) * ncx + tx]) continue;
+      cp.coarse_list.push_back(uint32_t(tx) | (uint32_t(ty) << 16));
+      // pyr_coarse's regions: the tile at level 1, then per level the tile's footprint plus the
+      // upsample halo (the kernel's own recursion), as level-0 pixels.
+      int ax = tx * t1, ay = ty * t1, bx = std::min(ax + t1, lw1), by = std::min(ay + t1, lh1);
+      int f0x = ax << 1, f0y = ay << 1, f1x = bx << 1, f1y = by << 1;
+      for (int l = 2; l < L; ++l) {
+        ax >>= 1;
+        ay >>= 1;
+        bx = std::min(((bx - 1) >> 1) + 2, p.lw[l]);
+        by = std::min(((by - 1) >> 1) + 2, p.lh[l]);
+        f0x = std::min(f0x, ax << l);
+        f0y = std::min(f0y, ay << l);
+        f1x = std::max(f1x, bx << l);
+        f1y = std::max(f1y, by << l);
+      }
+      mark_down(f0x, f0y, f1x - 1, f1y - 1);
+    }
+  // Down tiles that meet a pyramid block's pixels: pyr_fine reads their kept level-0 pixels.
+  std::vector<uint8_t> keep0(size_t(ndx) * ndy, 0);
+  for (uint32_t f : cp.fine_list) {
+    const int i = int(f & 0xFFFFu), j = int(f >> 16);
+    const int x0 = std::max(cp.fx0 + 64 * i, wx0), x1 = std::min(cp.fx0 + 64 * i + 64, wx1) - 1;
+    const int y0 = std::max(cp.fy0 + 16 * j, wy0), y1 = std::min(cp.fy0 + 16 * j + 16, wy1) - 1;
+    for (int ty = y0 / td; ty <= y1 / td; ++ty)
+      for (int tx = x0 / td; tx <= x1 / td; ++tx) keep0[size_t(ty) * ndx + tx] = 1;
+  }
+  for (int ty = 0; ty < ndy; ++ty)
+    for (int tx = 0; tx < ndx; ++tx) {
+      if (!dmark[size_t(ty) * ndx + tx]) continue;
+      cp.down_list.push_back(uint32_t(tx) | (uint32_t(ty) << 16) | (keep0[size_t(ty) * ndx + tx] ? 0x80000000u : 0u));
+    }
+  cp.usable = cp.copy_blocks + cp.empty_blocks > 0 && ndx < 0x8000 && ndy < 0x8000 && ncx < 0x8000 &&
+              ncy < 0x8000 && cp.nfx < 0x8000 && cp.nfy < 0x8000;
+}
+
 void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
   cp = CopyPlan{};
   const int L = p.levels, n = p.n;
@@ -135,70 +205,15 @@ void plan_copy_blocks(const Plan& p, int td, int t1, CopyPlan& cp) {
       }
     }
 
-  // Level-1 tiles whose R^1 the pyramid blocks read (pyr_fine's 33 x 9 level-1 tile from
-  // (bx0 / 2, by0 / 2), coordinates clamped to the level), and level-0 tiles whose G^l levels (or
-  // kept level-0 pixels) pyr_fine and pyr_coarse read.
-  const int lw1 = p.lw[1], lh1 = p.lh[1];
-  const int ncx = (lw1 + t1 - 1) / t1, ncy = (lh1 + t1 - 1) / t1;
-  const int ndx = (bw + td - 1) / td, ndy = (bh + td - 1) / td;
-  cp.dense_coarse = (long long)ncx * ncy;
-  cp.dense_down = (long long)ndx * ndy;
-  std::vector<uint8_t> cmark(size_t(ncx) * ncy, 0), dmark(size_t(ndx) * ndy, 0);
-  const auto mark_down = [&](int lx0, int ly0, int lx1, int ly1) {  // level-0 pixels, inclusive
-    lx0 = std::max(lx0, 0);
-    ly0 = std::max(ly0, 0);
-    lx1 = std::min(lx1, bw - 1);
-    ly1 = std::min(ly1, bh - 1);
-    for (int ty = ly0 / td; ty <= ly1 / td; ++ty)
-      for (int tx = lx0 / td; tx <= lx1 / td; ++tx) dmark[size_t(ty) * ndx + tx] = 1;
-  };
-  for (uint32_t f : cp.fine_list) {
-    const int bx0 = cp.fx0 + 64 * int(f & 0xFFFFu), by0 = cp.fy0 + 16 * int(f >> 16);
-    const int tx0 = bx0 >> 1, ty0 = by0 >> 1;
-    const int tx1 = std::min(tx0 + 32, lw1 - 1), ty1 = std::min(ty0 + 8, lh1 - 1);
-    for (int ty = ty0 / t1; ty <= ty1 / t1; ++ty)
-      for (int tx = tx0 / t1; tx <= tx1 / t1; ++tx) cmark[size_t(ty) * ncx + tx] = 1;
-    mark_down(2 * tx0, 2 * ty0, 2 * tx1 + 1, 2 * ty1 + 1);  // G^1 taps; the block's own pixels lie inside
-  }
-  for (int ty = 0; ty < ncy; ++ty)
-    for (int tx = 0; tx < ncx; ++tx) {
-      if (!cmark[size_t(ty) * ncx + tx]) continue;
-      cp.coarse_list.push_back(uint32_t(tx) | (uint32_t(ty) << 16));
-      // pyr_coarse's regions: the tile at level 1, then per level the tile's footprint plus the
-      // upsample halo (the kernel's own recursion), as level-0 pixels.
-      int ax = tx * t1, ay = ty * t1, bx = std::min(ax + t1, lw1), by = std::min(ay + t1, lh1);
-      int f0x = ax << 1, f0y = ay << 1, f1x = bx << 1, f1y = by << 1;
-      for (int l = 2; l < L; ++l) {
-        ax >>= 1;
-        ay >>= 1;
-        bx = std::min(((bx - 1) >> 1) + 2, p.lw[l]);
-        by = std::min(((by - 1) >> 1) + 2, p.lh[l]);
-        f0x = std::min(f0x, ax << l);
-        f0y = std::min(f0y, ay << l);
-        f1x = std::max(f1x, bx << l);
-        f1y = std::max(f1y, by << l);
-      }
-      mark_down(f0x, f0y, f1x - 1, f1y - 1);
-    }
-  // Down tiles that meet a pyramid block's pixels: pyr_fine reads their kept level-0 pixels.
-  std::vector<uint8_t> keep0(size_t(ndx) * ndy, 0);
-  for (uint32_t f : cp.fine_list) {
-    const int i = int(f & 0xFFFFu), j = int(f >> 16);
-    const int x0 = std::max(cp.fx0 + 64 * i, wx0), x1 = std::min(cp.fx0 + 64 * i + 64, wx1) - 1;
-    const int y0 = std::max(cp.fy0 + 16 * j, wy0), y1 = std::min(cp.fy0 + 16 * j + 16, wy1) - 1;
-    for (int ty = y0 / td; ty <= y1 / td; ++ty)
-      for (int tx = x0 / td; tx <= x1 / td; ++tx) keep0[size_t(ty) * ndx + tx] = 1;
-  }
-  for (int ty = 0; ty < ndy; ++ty)
-    for (int tx = 0; tx < ndx; ++tx) {
-      if (!dmark[size_t(ty) * ndx + tx]) continue;
-      cp.down_list.push_back(uint32_t(tx) | (uint32_t(ty) << 16) | (keep0[size_t(ty) * ndx + tx] ? 0x80000000u : 0u));
-    }
   cp.support_mark = std::move(support_mark);
   cp.support_pitch = gx;
   cp.support_shift = L - 1;
-  cp.usable = cp.copy_blocks + cp.empty_blocks > 0 && ndx < 0x8000 && ndy < 0x8000 && ncx < 0x8000 &&
-              ncy < 0x8000 && cp.nfx < 0x8000 && cp.nfy < 0x8000;
+  list_tiles(p, td, t1, cp);
+}
+
+void replan_tiles(const Plan& p, int td, int t1, const CopyPlan& from, CopyPlan& cp) {
+  cp = from;
+  if (!from.block_class.empty()) list_tiles(p, td, t1, cp);
 }
 
 void rgb_canvas_plane(Plan& p, const CopyPlan& c) {
@@ -221,18 +236,26 @@ void rgb_canvas_plane(Plan& p, const CopyPlan& c) {
       const int y0 = std::max(c.fy0 + 16 * j, wy0), y1 = std::min(c.fy0 + 16 * j + 16, wy1);
       const int label = p.mask0[size_t(y0) * p.lw[0] + x0];
       const GatherPlane& s = p.slots[p.rule == kRuleTwo ? (label == 1 ? 0 : 1) : label];
-      for (int y = y0; y < y1; ++y)
-        for (int x = x0; x < x1; ++x) {
-          const size_t d = size_t(y + p.blend.y) * p.canvas_w + (x + p.blend.x);
-          if (!s.rect.contains(x, y)) {
-            g.owner[d] = kNoOwner;
-            g.map[d] = kNoEntry;
-            continue;
-          }
-          const size_t q = size_t(y - s.rect.y) * s.rect.w + (x - s.rect.x);
-          g.owner[d] = s.map[q] == kNoEntry ? kNoOwner : (s.owner.empty() ? uint8_t(s.default_owner) : s.owner[q]);
-          g.map[d] = s.map[q];
-        }
+      // Row by row: the slot's entries inside its plane, none outside.
+      const int sx0 = std::min(std::max(x0, s.rect.x), x1), sx1 = std::max(std::min(x1, s.rect.x + s.rect.w), sx0);
+      for (int y = y0; y < y1; ++y) {
+        const size_t d = size_t(y + p.blend.y) * p.canvas_w + p.blend.x;
+        uint32_t* map = &g.map[d];
+        uint8_t* owner = &g.owner[d];
+        const bool in = y >= s.rect.y && y < s.rect.y + s.rect.h;
+        const int a = in ? sx0 : x1, b = in ? sx1 : x1;
+        std::fill(map + x0, map + a, kNoEntry);
+        std::fill(map + b, map + x1, kNoEntry);
+        std::fill(owner + x0, owner + a, kNoOwner);
+        std::fill(owner + b, owner + x1, kNoOwner);
+        if (a >= b) continue;
+        const size_t q = size_t(y - s.rect.y) * s.rect.w + (a - s.rect.x);
+        std::copy(&s.map[q], &s.map[q] + (b - a), map + a);
+        if (s.owner.empty())
+          for (int x = a; x < b; ++x) owner[x] = map[x] == kNoEntry ? kNoOwner : uint8_t(s.default_owner);
+        else
+          for (int x = a; x < b; ++x) owner[x] = map[x] == kNoEntry ? kNoOwner : s.owner[q + (x - a)];
+      }
     }
 }
 

@@ -74,6 +74,10 @@ struct CopyPlan {
 // short dyadic fractions), and float pixels. RGB8: any blend region of two or more levels.
 void plan_copy_blocks(const Plan& p, int tile_down, int tile_coarse, CopyPlan& out);
 
+// The same plan for another down-tile edge (`from`: plan_copy_blocks' result): the blocks' classes do not
+// depend on it, only the lists of tiles do.
+void replan_tiles(const Plan& p, int tile_down, int tile_coarse, const CopyPlan& from, CopyPlan& out);
+
 // RGB8: writes the copy blocks' slot entries into the canvas plane (made here where the
 // configuration has none).
 void rgb_canvas_plane(Plan& p, const CopyPlan& c);
