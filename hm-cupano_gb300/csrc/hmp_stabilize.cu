@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
 
 // Windows of 5 to 21 pixels: a CTA per 64 x 64 tile of the frame (and 128 features), one to a thread, the
 // tile of `prev` (with the window's halo and the gradients') and of `next` (with the window's halo
-// and kFlowMargin pixels of motion) in shared memory. Features of a warp sit at scattered places, so
+// and flow_margin pixels of motion) in shared memory. Features of a warp sit at scattered places, so
 // their taps are 4-byte accesses at unrelated addresses: from L1 each costs a wavefront per lane,
 // from shared memory one per bank conflict. Both tiles have a pitch of 96 words (a multiple of 32),
 // so a tap's bank depends on its column alone, and the tile's features are dealt out to the warps
@@ -397,9 +397,12 @@ __global__ void __launch_bounds__(256) flow_kernel(const float* __restrict__ pre
 // features by tile.
 constexpr int kFlowTile = 64, kFlowPitch = 96, kFlowThreads = 128;
 constexpr int kFlowMinHalf = 2, kFlowMaxHalf = 10, kFlowFewFar = 6;
-__host__ __device__ constexpr int flow_margin(int half) { return (kFlowPitch - kFlowTile) / 2 - half; }  // so `next` is 96 x 96
+// Pixels of motion staged around a tile of `next`, so that it is 96 x 96: 9 at window 15, 6 at 21.
+__host__ __device__ constexpr int flow_margin(int half) { return (kFlowPitch - kFlowTile) / 2 - half; }
 __host__ __device__ constexpr int flow_prev_rows(int half) { return kFlowTile + 2 * half + 2; }
-__host__ __device__ constexpr int flow_smem(int half) { return (flow_prev_rows(half) + kFlowPitch) * kFlowPitch * int(sizeof(float)); }
+__host__ __device__ constexpr int flow_smem(int half) {
+  return (flow_prev_rows(half) + kFlowPitch) * kFlowPitch * int(sizeof(float));
+}
 
 __device__ __forceinline__ void copy_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src));
@@ -737,7 +740,8 @@ __global__ void __launch_bounds__(kFlowThreads, 3)
       }
       if (!__any_sync(0xFFFFFFFFu, need)) break;
       // A warp's windows beyond the staged part wait for those inside it, where they are more than a few: then
-      // they are summed together, not beside one of the others pass after pass.
+      // they are summed together, not beside one of the others pass after pass (3840x2160, 12 px: 1640 -> 1540 us
+      // a call). A few outliers are not worth the others' wait: 3 to 4 % of the flow at window 21 and 3 px.
       const bool near1 = abs(rx - cx) <= M && abs(ry - cy) <= M;
       const unsigned far_lanes = __ballot_sync(0xFFFFFFFFu, need && !near1);
       const bool defer = __any_sync(0xFFFFFFFFu, need && near1) && __popc(far_lanes) > kFlowFewFar;
@@ -1062,12 +1066,11 @@ struct hmp_stabilizer {
   Motion* motion = nullptr;
   float* temp = nullptr;  // an in-place warp's output before the copy back
   int tiles_x = 0, tiles = 0;  // flow tiles of the frame
-  FlowItems items{};           // `cnt` and, after it, `n_items` are cleared together
+  FlowItems items{};           // one allocation: items, order, at, cnt and n_items (cleared together)
   ~hmp_stabilizer() {
-    for (void* p : {static_cast<void*>(resp), static_cast<void*>(corner_bits), static_cast<void*>(row_cnt), static_cast<void*>(row_off),
-                    static_cast<void*>(xy), static_cast<void*>(flow), static_cast<void*>(motion),
-                    static_cast<void*>(temp), static_cast<void*>(items.cnt), static_cast<void*>(items.at),
-                    static_cast<void*>(items.order), static_cast<void*>(items.items)})
+    for (void* p : {static_cast<void*>(resp), static_cast<void*>(corner_bits), static_cast<void*>(row_cnt),
+                    static_cast<void*>(row_off), static_cast<void*>(xy), static_cast<void*>(flow),
+                    static_cast<void*>(motion), static_cast<void*>(temp), static_cast<void*>(items.items)})
       if (p) cudaFree(p);
   }
   int most_items() const { return tiles + cap / kFlowThreads; }
@@ -1092,8 +1095,9 @@ void launch_flow_tile(const hmp_stabilizer& st, const float* prev, const float* 
 
 using FlowTileLaunch = void (*)(const hmp_stabilizer&, const float*, const float*, cudaStream_t);
 constexpr FlowTileLaunch kFlowTileLaunch[kFlowMaxHalf + 1] = {
-    nullptr,             nullptr,             launch_flow_tile<2>, launch_flow_tile<3>, launch_flow_tile<4>, launch_flow_tile<5>,
-    launch_flow_tile<6>, launch_flow_tile<7>, launch_flow_tile<8>, launch_flow_tile<9>, launch_flow_tile<10>};
+    nullptr,             nullptr,             launch_flow_tile<2>, launch_flow_tile<3>, launch_flow_tile<4>,
+    launch_flow_tile<5>, launch_flow_tile<6>, launch_flow_tile<7>, launch_flow_tile<8>, launch_flow_tile<9>,
+    launch_flow_tile<10>};
 
 template <int HALF = kFlowMaxHalf>
 cudaError_t flow_tile_init() {
@@ -1134,11 +1138,15 @@ HMP_API hmp_status hmp_stabilizer_create(int width, int height, int max_features
   if (e == cudaSuccess) e = cudaMalloc(&st->flow, size_t(std::max(st->cap, 1)) * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&st->motion, sizeof(Motion));
   if (e == cudaSuccess) e = cudaMalloc(&st->temp, px * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&st->items.cnt, size_t(st->tiles + 2) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&st->items.at, size_t(st->tiles) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&st->items.order, size_t(std::max(st->cap, 1)) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&st->items.items, size_t(st->most_items()) * sizeof(int2));
-  if (e == cudaSuccess) st->items.n_items = st->items.cnt + st->tiles;
+  if (e == cudaSuccess)
+    e = cudaMalloc(&st->items.items, size_t(st->most_items()) * sizeof(int2) +
+                                         (size_t(std::max(st->cap, 1)) + 2 * size_t(st->tiles) + 2) * sizeof(int));
+  if (e == cudaSuccess) {
+    st->items.order = reinterpret_cast<int*>(st->items.items + st->most_items());
+    st->items.at = st->items.order + std::max(st->cap, 1);
+    st->items.cnt = st->items.at + st->tiles;
+    st->items.n_items = st->items.cnt + st->tiles;
+  }
   if (e == cudaSuccess) e = flow_tile_init();
   if (e == cudaSuccess) e = cudaMemset(st->motion, 0, sizeof(Motion));
   if (e != cudaSuccess) {
