@@ -29,7 +29,8 @@
 //   * every source pixel in a copy block's support must have alpha != 0 (checked on the device:
 //     by the gather over the blend region, for the pixels it copies and those outside the write
 //     rect, and by pyr_fine (two images: by pyr_down, which reads them earlier) for the
-//     pyramid-block pixels inside a support, the only others a support holds; any alpha 0 gates on the fallback launches, which recompute the write rect).
+//     pyramid-block pixels inside a support, the only others a support holds; any alpha 0 gates on
+//     the fallback launches, which recompute the write rect).
 // RGB8 frames have no alpha and no validity: an unmapped pixel is 0 and counts like any other, so a
 // block is a copy wherever the labels of its supports are one image's, the copied pixel is that
 // slot's level-0 pixel (0 where it has none), and nothing is checked per frame. The canvas plane

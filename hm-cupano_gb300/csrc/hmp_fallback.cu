@@ -3,11 +3,11 @@
 // Copy blocks are exact only while every source pixel in their supports has alpha != 0; the canvas
 // gather and pyr_fine (two images: pyr_down) check that and set a flag. Most calls leave it clear, so
 // the fallback must cost as little as possible then: one thread of fallback_gate_kernel reads the flag
-// after the kernels that set it (two images: beside the rest of the chain) and returns. When it is set, the thread clears it and tail-launches the
-// dense chain (pyr_down, pyr_coarse, pyr_fine over every tile of the write rect, the instantiations
-// the plain path uses), which recomputes the whole write rect after the gather wrote its copy
-// blocks; tail launches run in order, each after the one before and after this grid, and the
-// caller's stream continues only after the last.
+// after the kernels that set it (two images: beside the rest of the chain) and returns. When it is set,
+// the thread clears it and tail-launches the dense chain (pyr_down, pyr_coarse, pyr_fine over every tile
+// of the write rect, the instantiations the plain path uses), which recomputes the whole write rect after
+// the gather wrote its copy blocks; tail launches run in order, each after the one before and after this
+// grid, and the caller's stream continues only after the last.
 //
 // Device-side launches need relocatable device code, which raises the pyramid kernels' registers
 // markedly, so this unit (-rdc=true) holds its own copies of the kernels (hmp_pyramid_kernels.cuh)

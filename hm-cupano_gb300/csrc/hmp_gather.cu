@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(256, 4) canvas_gather_packed_kernel(const __gr
 // Resolves one plane's packed entries (raw.map) for the frames' geometry (res, same layout):
 // owner o < n and (sx, sy) inside image o give o << 29 | (sy * pitch / 4 + sx); anything else
 // kOffZero, or kOffOpaque under the soft-seam rule when the owner is valid and sx is not the
-// 65535 sentinel. rgb: byte offsets of three-byte pixels. (Frames hold fewer than kOffMask - 1 pixels, so no offset meets a fill code.)
+// 65535 sentinel. rgb: byte offsets of three-byte pixels. (Frames hold fewer than kOffMask - 1 pixels, or
+// bytes, so no offset meets a fill code.)
 __global__ void __launch_bounds__(kSegPixels) resolve_plane_kernel(const __grid_constant__ PlaneDev raw, uint32_t* res,
                                                                    uint8_t* seg_owner, int seg_pitch,
                                                                    const __grid_constant__ SrcSet S, int n, int opaque,

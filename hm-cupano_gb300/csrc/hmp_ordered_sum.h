@@ -31,7 +31,7 @@ struct OrderedRun {
 
 // The pair of one element, r = x / u (exact: u is a power of two). False: too large, or not finite.
 // Adding 1.5 * 2^23 leaves r's nearest integer, ties to even, in the low bits of the sum (additions
-// only: a conversion costs eight of them).
+// only: a conversion issues at a quarter of their rate).
 HMP_HD bool ordered_element(float r, OrderedRun& e) {
   constexpr float kMagic = 12582912.0f;
   if (!(fabsf(r) < 4194304.0f)) return false;

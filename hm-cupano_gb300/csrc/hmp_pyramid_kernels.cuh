@@ -104,11 +104,11 @@ __device__ __forceinline__ Store* level_of(const PyrArgs& a, int k, int l, int b
 }
 
 // Gaussian levels 1..L-1 of every slot for one TD x TD level-0 tile (TD a multiple of 2^(L-1),
-// so no level needs a neighbouring tile). Level 0 is gathered into shared memory (gather_slot). One pass then reduces each 4x4 pixel block to its four level-1 pixels
-// (kept in registers and stored to HBM) and their level-2 pixel; deeper levels reduce the
-// previous level in shared memory (levels 3, 5 reuse the level-0 buffer). Every level >= 1 goes
-// to HBM. A slot whose plane misses the tile produces zeros, which its level buffers already
-// hold, so it is skipped entirely.
+// so no level needs a neighbouring tile). Level 0 is gathered into shared memory (gather_slot). One
+// pass then reduces each 4x4 pixel block to its four level-1 pixels (kept in registers and stored to
+// HBM) and their level-2 pixel; deeper levels reduce the previous level in shared memory (levels 3, 5
+// reuse the level-0 buffer). Every level >= 1 goes to HBM. A slot whose plane misses the tile produces
+// zeros, which its level buffers already hold, so it is skipped entirely.
 // Programmatic dependent launch: pyr_coarse and pyr_fine are launched with programmatic stream
 // serialization, so their CTAs can be scheduled as the kernel before them on the stream drains
 // (its CTAs trigger implicitly at exit; an explicit early trigger measured slower beside the
@@ -224,7 +224,8 @@ __device__ __forceinline__ const uchar4* slot_src_dyn(const PyrArgs& a, int k, i
 // pyramid-block pixel. (Three and more images: pyr_fine, which reads only the label's pixel.)
 // Before (entries and pixels through cp.async, the frame looked up per pixel) the kernels spent their
 // issue slots on addresses: eight images 9000x2400, 1663 tiles, 64.4 -> 52.5 us; three 6000x1800 FP16,
-// 855 tiles, 32.8 -> 31.2; two 8500x3300, 318 tiles, 18.6 -> 17.2 (alone, cold).
+// 855 tiles, 32.8 -> 31.2; two 8500x3300, 318 tiles, 18.6 -> 17.2 without the alpha check (alone, cold;
+// on a rig of 343 tiles 20.1 before and 24.5 now with it, which the gate beside the chain repays).
 template <int TD, bool kCheck>
 __device__ __forceinline__ void gather_slot(const PyrArgs& a, int k, uint32_t* pk, int X0, int Y0, int b, bool opaque,
                                             bool keep) {

@@ -618,8 +618,8 @@ __global__ void __launch_bounds__(256) rgb_fine_kernel(const __grid_constant__ P
 // assembled into words in shared memory (each word takes two neighbouring pixels) so that the canvas
 // is written in full lines; the words at a segment's ends, and those with a pixel the pyramid writes,
 // are stored byte by byte. kPacked: frames past the offsets' range, from the packed entries.
-// HBM-bound: 4 (entry) + 3 + 3 bytes a pixel. 8500x3300 (27 Mpx of it): 181 -> 61 us alone,
-// 4.4 TB/s; what is left is the issue of about 45 instructions a pixel.
+// 4 (entry) + 3 + 3 bytes a pixel; bound by the issue of 57 instructions a pixel (70 % of the issue slots).
+// 8500x3300 (27 Mpx of it): 181 -> 61 us alone, 4.4 TB/s.
 constexpr uint32_t kRgbSkip = 0x80000000u;  // a staged pixel that is not stored
 
 template <bool kPacked>
@@ -767,7 +767,7 @@ cudaError_t rgb_init() {
   cudaFuncSetAttribute(rgb_coarse_kernel<kRuleTwo, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
   cudaFuncSetAttribute(rgb_coarse_kernel<kRuleThree, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
   cudaFuncSetAttribute(rgb_coarse_kernel<kRuleNway, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
-  // Eight slots' G^1 tiles and the staged rows: 46 KB, past the default limit with the static part.
+  // Eight slots' G^1 tiles and the staged rows: 46 KB, close to the default limit.
   cudaFuncSetAttribute(rgb_fine_kernel<kRuleTwo>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax - 8192);
   cudaFuncSetAttribute(rgb_fine_kernel<kRuleThree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax - 8192);
   cudaFuncSetAttribute(rgb_fine_kernel<kRuleNway>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax - 8192);

@@ -838,7 +838,8 @@ struct hmp_stitcher {
     return S;
   }
 
-  // float4 / float3 pixels: the canvas outside the write rect, then the pyramid level by level, all on the caller's stream (hmp_generic.cu).
+  // float4 / float3 pixels: the canvas outside the write rect, then the pyramid level by level, all on the
+  // caller's stream (hmp_generic.cu).
   hmp_status process_generic(const hmp::SrcSet& S, const hmp_image* canvas, cudaStream_t s) {
     const hmp::Plan& p = plan;
     hmp::CanvasDev C;
