@@ -133,7 +133,7 @@ __device__ __forceinline__ bool stage_tile(float4* t, const T* low, int lw, int 
   bool solid = true;
   for (int i = threadIdx.y * 32 + threadIdx.x; i < area; i += 256) {
     const int sx = reflect101(U0 + i % pitch, lw), sy = reflect101(V0 + i / pitch, lh);
-    const float4 v = load_level(low + (long long)sy * lw + sx);
+    const float4 v = load_dep(low + (long long)sy * lw + sx);
     t[i] = v;
     solid = solid && v.w != 0.f;
   }
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) b5_down_kernel(const __grid_constant__ Py
       const Store* src = static_cast<const Store*>(a.G[k0 + g][l]) + (long long)b * iw * ih;
 #pragma unroll
       for (int u = 0; u < kB5Per; ++u)
-        if (tid + 256 * u < kB5SrcArea) t[g][tid + 256 * u] = load_level(src + so[u]);
+        if (tid + 256 * u < kB5SrcArea) t[g][tid + 256 * u] = load_dep(src + so[u]);
     }
     unsigned hole = 0;  // images whose tile has a pixel without alpha
 #pragma unroll
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(256) b5_up_kernel(const __grid_constant__ PyrA
   float al[NMAX], m[NMAX];
 #pragma unroll
   for (int k = 0; k < NMAX; ++k) {
-    g[k] = k < n && inside ? load_level(g_of<NMAX, Store>(a, k, l, b) + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    g[k] = k < n && inside ? load_dep(g_of<NMAX, Store>(a, k, l, b) + o) : make_float4(0.f, 0.f, 0.f, 0.f);
     m[k] = k < K && inside ? __ldg(a.maskL[l] + o * K + k) : 0.f;
   }
   const int U0 = (X0 >> 1) - 1, V0 = (Y0 >> 1) - 1;

@@ -388,4 +388,26 @@ __device__ __forceinline__ float4 blend_level0(int n, const float4* lap, int v) 
   }
 }
 
+// A level pixel that the kernel before wrote, read by a kernel that starts before that one is done and waits
+// inside (griddepcontrol.wait): an ordinary load, in order with the wait. (__ldg promises data that is
+// constant for the kernel's whole life.) Of global memory by name: through a plain pointer the eight-image
+// 9000x2400 frame took 195.7 us instead of 194.4, a small two-image one 33.4 instead of 33.0.
+__device__ __forceinline__ float4 load_dep(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_dep(const half4* p) {
+  uint2 raw;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];\n" : "=r"(raw.x), "=r"(raw.y) : "l"(p));
+  const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+  const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+  return make_float4(fa.x, fa.y, fb.x, fb.y);
+}
+__device__ __forceinline__ uint32_t load_dep(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p));
+  return v;
+}
+
 }  // namespace hmp

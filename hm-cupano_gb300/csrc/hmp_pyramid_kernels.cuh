@@ -114,10 +114,10 @@ __device__ __forceinline__ Store* level_of(const PyrArgs& a, int k, int l, int b
 // (its CTAs trigger implicitly at exit; an explicit early trigger measured slower beside the
 // canvas gather, the waiting CTAs holding SM resources). griddepcontrol.wait returns once that
 // kernel has completed and its writes are visible (at once after a normal launch).
-// What those kernels write is read with ordinary loads only. __ldg promises data that is constant for
+// What those kernels write is read with ordinary loads only (load_dep). __ldg promises data that is constant for
 // the kernel's whole life, which here begins before the data is written, so such a load may be made
 // ahead of the wait. In the gated fallback, whose kernels start together, that gave pixels of an earlier
-// frame (three images, captured, the first replay that fell back). Ordinary loads cost nothing measurable.
+// frame (three images, captured, the first replay that fell back).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // The gated fallback launches (copy-block mode) let their dependents start at once: a fallback CTA
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(256) pyr_coarse_kernel(const __grid_constant__
         m[q] = q < K ? __ldg(a.maskL[1] + o1 * K + q) : 0.f;
   #pragma unroll
       for (int k = 0; k < NMAX; ++k) {
-        g1[k] = ((amask >> k) & 1u) ? load_level(static_cast<const Store*>(a.G[k][1]) + (long long)b * lw1 * lh1 + o1)
+        g1[k] = ((amask >> k) & 1u) ? load_dep(static_cast<const Store*>(a.G[k][1]) + (long long)b * lw1 * lh1 + o1)
                                     : make_float4(0.f, 0.f, 0.f, 0.f);
         al[k] = g1[k].w;
       }
@@ -919,7 +919,7 @@ __global__ void __launch_bounds__(256) pyr_coarse_n_kernel(const __grid_constant
       if (px >= lw1 || py >= lh1) continue;
       const long long o1 = (long long)py * lw1 + px;
       const auto pix = [&](int ci) {
-        return load_level(static_cast<const Store*>(a.G[(list >> (4 * ci)) & 15u][1]) + boff + o1);
+        return load_dep(static_cast<const Store*>(a.G[(list >> (4 * ci)) & 15u][1]) + boff + o1);
       };
       const auto lap = [&](int ci, float4 g) {
         if (has2) {
@@ -1069,7 +1069,7 @@ __global__ void __launch_bounds__(256) pyr_fine_kernel(const __grid_constant__ P
             const int rx = x - P.x0, ry = y - P.y0;
             ent[u][k] = 0u;
             if (live[u] && ((amask >> k) & 1u) && (unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-              ent[u][k] = a.P0[k][(long long)b * P.w * P.h + (long long)ry * P.w + rx];
+              ent[u][k] = load_dep(a.P0[k] + (long long)b * P.w * P.h + (long long)ry * P.w + rx);
           } else if (live[u] && ((amask >> k) & 1u)) {
             slot_lookup(a.slot[k], k, x, y, own[u][k], ent[u][k]);
           }
@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(256) pyr_fine_n_kernel(const __grid_constant__
           const PlaneDev& P = a.slot[v[q]];
           const int rx = x - P.x0, ry = y - P.y0;
           if ((unsigned)rx < (unsigned)P.w && (unsigned)ry < (unsigned)P.h)
-            p[q] = a.P0[v[q]][(long long)b * P.w * P.h + (long long)ry * P.w + rx];
+            p[q] = load_dep(a.P0[v[q]] + (long long)b * P.w * P.h + (long long)ry * P.w + rx);
         }
       }
       if (a.alpha_flag != nullptr) {  // copy-block mode, as in pyr_fine_kernel

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(256) rgb_coarse_kernel(const __grid_constant__
     const int px = X1 + 2 * ((i % CLS) % HALF) + ((i / CLS) & 1), py = Y1 + 2 * ((i % CLS) / HALF) + ((i / CLS) >> 1);
     own1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (hot1[p] < n && ((cmap >> (4 * hot1[p])) & 15u) < 15u)
-      own1[p] = load_level(static_cast<const float4*>(a.G[hot1[p]][1]) + boff + (long long)py * lw1 + px);
+      own1[p] = load_dep(static_cast<const float4*>(a.G[hot1[p]][1]) + boff + (long long)py * lw1 + px);
   }
   cp_async_commit_wait_all();
   __syncthreads();
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(256) rgb_coarse_kernel(const __grid_constant__
     const bool ox = (px & 1) != 0, oy = (py & 1) != 0;
     const auto lap = [&](int ci) {
       const int k = (list >> (4 * ci)) & 15u;
-      const float4 g = k == hot1[p] ? own1[p] : load_level(static_cast<const float4*>(a.G[k][1]) + boff + o);
+      const float4 g = k == hot1[p] ? own1[p] : load_dep(static_cast<const float4*>(a.G[k][1]) + boff + o);
       float3 r = make_float3(g.x, g.y, g.z);
       if (has2) {
         const float3 u = rgb_up(g2 + ci * CAP2, un, dx, dy, ox, oy);
